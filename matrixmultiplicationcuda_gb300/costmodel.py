@@ -80,7 +80,7 @@ class MLP:
         import torch
         X, T, mask = X.contiguous(), T.contiguous(), mask.contiguous()
         g = torch.empty_like(self.params)
-        loss = torch.zeros(1, dtype=torch.float32, device=self.device)
+        loss = torch.empty(1, dtype=torch.float32, device=self.device)
         check(lib().spmm_mlp_backward(ctypes.byref(self.s), _vp(self.params), _vp(X), _vp(T), _vp(mask),
                                       X.shape[0], _vp(g), _vp(loss), _vp(self._work(X.shape[0])),
                                       stream_handle(stream)))
