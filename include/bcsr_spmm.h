@@ -205,6 +205,15 @@ spmm_status spmm_dense_to_bcsr_count(const void* A, int M, int K, int lda, int b
                                      int* row_ptr, long long* nnzb_out, void* stream);
 spmm_status spmm_dense_to_bcsr_fill(const void* A, int M, int K, int lda, int bR, int bC,
                                     const int* row_ptr, int* col_idx, void* vals, void* stream);
+/* The same two steps with a workspace between them: count_masks also writes
+ * which blocks it found nonzero (spmm_dense_to_bcsr_mask_words 32-bit words,
+ * device memory), and fill_masks reads only those blocks of A instead of all of
+ * A again. A must not change in between. NULL masks run the steps above. */
+long long spmm_dense_to_bcsr_mask_words(int M, int K, int bR, int bC);
+spmm_status spmm_dense_to_bcsr_count_masks(const void* A, int M, int K, int lda, int bR, int bC, int* row_ptr,
+                                           unsigned* masks, long long* nnzb_out, void* stream);
+spmm_status spmm_dense_to_bcsr_fill_masks(const void* A, int M, int K, int lda, int bR, int bC, const int* row_ptr,
+                                          const unsigned* masks, int* col_idx, void* vals, void* stream);
 
 /* ---- generators on the GPU ------------------------------------------------------
  * The host generators' counter-based streams (bcsr_spmm_host.h), evaluated on

@@ -116,6 +116,10 @@ _SIGS = {
     "sparseMatrixMulTensorAdaptive32x16_launch": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_uint, c_uint, c_uint, c_uint, c_vp]),
     "sparseMatrixMulTensorAdaptive64x16_launch": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_uint, c_uint, c_uint, c_uint, c_vp]),
     "spmm_dense_to_bcsr_count": (c_int, [c_vp, c_int, c_int, c_int, c_int, c_int, c_vp, ctypes.POINTER(c_ll), c_vp]),
+    "spmm_dense_to_bcsr_mask_words": (c_ll, [c_int, c_int, c_int, c_int]),
+    "spmm_dense_to_bcsr_count_masks": (c_int, [c_vp, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp,
+                                               ctypes.POINTER(c_ll), c_vp]),
+    "spmm_dense_to_bcsr_fill_masks": (c_int, [c_vp, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp, c_vp]),
     "spmm_dense_to_bcsr_fill": (c_int, [c_vp, c_int, c_int, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp]),
     "spmm_quantize": (c_int, [c_vp, c_size, c_int, c_int, c_vp, c_vp, c_vp, c_vp]),
     "spmm_batch_plan_create": (c_int, [ctypes.POINTER(Problem), c_int, ctypes.POINTER(Config), ctypes.POINTER(c_vp)]),

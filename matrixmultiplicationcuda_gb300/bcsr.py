@@ -310,15 +310,19 @@ def dense_to_bcsr(A_half, bR=16, bC=16, stream=None):
     lda = A_half.stride(0)
     MB = M // bR
     rp = torch.empty(MB + 1, dtype=torch.int32, device=A_half.device)
+    masks = torch.empty(max(lib().spmm_dense_to_bcsr_mask_words(M, K, bR, bC), 0), dtype=torch.int32,
+                        device=A_half.device)
+    if stream is not None:
+        masks.record_stream(stream)   # its last reader runs there
     nnzb = ctypes.c_longlong(0)
     s = stream_handle(stream)
-    check(lib().spmm_dense_to_bcsr_count(_ptr(A_half), M, K, lda, bR, bC, _ptr(rp),
-                                         ctypes.byref(nnzb), s))
+    check(lib().spmm_dense_to_bcsr_count_masks(_ptr(A_half), M, K, lda, bR, bC, _ptr(rp), _ptr(masks),
+                                               ctypes.byref(nnzb), s))
     ci = torch.empty(max(nnzb.value, 0), dtype=torch.int32, device=A_half.device)
     vals = torch.empty(max(nnzb.value, 0) * bR * bC, dtype=torch.float16, device=A_half.device)
     if nnzb.value:
-        check(lib().spmm_dense_to_bcsr_fill(_ptr(A_half), M, K, lda, bR, bC, _ptr(rp), _ptr(ci),
-                                            _ptr(vals), s))
+        check(lib().spmm_dense_to_bcsr_fill_masks(_ptr(A_half), M, K, lda, bR, bC, _ptr(rp), _ptr(masks), _ptr(ci),
+                                                  _ptr(vals), s))
     return rp, ci, vals
 
 

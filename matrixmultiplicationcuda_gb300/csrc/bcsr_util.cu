@@ -3,6 +3,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
+#include <algorithm>
 #include <cstring>
 #include "internal.h"
 #include "ptx.cuh"
@@ -20,32 +21,32 @@ __device__ __forceinline__ bool any_nonzero_h8(uint4 v) {
   return nz(v.x) || nz(v.y) || nz(v.z) || nz(v.w);
 }
 
-// One CTA per block row. A warp covers 32 lanes x 16 bytes of a row of A, i.e.
-// 256 / bC whole blocks (bC / 8 lanes each), and walks the bR rows of the block
-// row, so every load is a coalesced 512-byte row segment.
-// Pass 1 (FILL = false) writes the block count of the row to counts[br].
-// Pass 2 (FILL = true) writes col_idx and copies the kept blocks, in ascending
-// block-column order, starting at row_ptr[br] (formats/BCSRMatrix.cu:55-71).
-template <bool FILL>
-__global__ void __launch_bounds__(kConvThreads)
-    k_dense_to_bcsr(const uint16_t* __restrict__ A, long long lda, int bR, int bC, int KB,
-                    int* __restrict__ counts, const int* __restrict__ row_ptr,
-                    int* __restrict__ col_idx, uint16_t* __restrict__ vals) {
-  extern __shared__ uint32_t sm[];  // masks[ngroups], offsets[ngroups]
+// Which blocks hold a nonzero. A warp covers 32 lanes x 16 bytes of a row of A,
+// i.e. a group of 32 / (bC / 8) whole blocks (bC / 8 lanes each), and walks the
+// bR rows of the block row, so every load is a coalesced 512-byte row segment, 8
+// in flight a lane. Output, one of: masks, one word per group, bit b set when
+// block b of the group is kept (grid: block rows x runs of groups); or counts,
+// the kept blocks of each row (one CTA a row).
+// DRAM-bound. With masks the CTAs are small, so that the SMs finish together:
+// one CTA a row gave an SM three or four of the 512 rows of an 8192^2 matrix in
+// 16-row blocks, and its 134 MB took 31-33 us (28 now, the copy rate allows 20).
+__global__ void __launch_bounds__(1024)
+    k_block_masks(const uint16_t* __restrict__ A, long long lda, int bR, int bC, int KB, int ngroups,
+                  uint32_t* __restrict__ masks, int* __restrict__ counts) {
   const int br = blockIdx.x;
   const int lpb = bC / 8;                 // lanes per block
   const int gblk = 32 / lpb;              // blocks per warp pass
-  const int ngroups = (KB + gblk - 1) / gblk;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-  uint32_t* masks = sm;
-  uint32_t* offs = sm + ngroups;
   __shared__ int row_total;
-  if (threadIdx.x == 0) row_total = 0;
-  __syncthreads();
-
+  if (counts) {
+    if (threadIdx.x == 0) row_total = 0;
+    __syncthreads();
+  }
+  grid_dep_launch_dependents();
+  grid_dep_wait();
   const uint16_t* arow = A + (long long)br * bR * lda;
   int local = 0;
-  for (int gi = warp; gi < ngroups; gi += nwarps) {
+  for (int gi = blockIdx.y * nwarps + warp; gi < ngroups; gi += nwarps * gridDim.y) {
     const int j = gi * gblk + lane / lpb;   // block column of this lane
     const int sub = lane % lpb;
     bool nz = false;
@@ -67,15 +68,111 @@ __global__ void __launch_bounds__(kConvThreads)
     for (int b = 0; b < gblk; ++b)
       if ((bal >> (b * lpb)) & lm) mask |= 1u << b;
     if (lane == 0) {
-      masks[gi] = mask;
+      if (masks) masks[(long long)br * ngroups + gi] = mask;
       local += __popc(mask);
     }
   }
-  if (!FILL) {
-    if (lane == 0 && local) atomicAdd(&row_total, local);
-    __syncthreads();
-    if (threadIdx.x == 0) counts[br] = row_total;
-    return;
+  if (!counts) return;
+  if (lane == 0 && local) atomicAdd(&row_total, local);
+  __syncthreads();
+  if (threadIdx.x == 0) counts[br] = row_total;
+}
+
+// The kept blocks, from the masks: a warp takes one group of one block row,
+// counts the row's kept blocks before it, writes their col_idx and copies them
+// in ascending block-column order from row_ptr[br] on (formats/BCSRMatrix.cu:
+// 55-71), four 512-byte pieces of blocks in flight. Only kept blocks of A are
+// read: 8192^2 at 5 % reads 6.7 MB of the 134 MB that the pass without masks
+// reads again.
+constexpr int kFillWarps = 8;
+__global__ void __launch_bounds__(32 * kFillWarps)
+    k_fill_masked(const uint16_t* __restrict__ A, long long lda, int bR, int bC, int ngroups,
+                  const uint32_t* __restrict__ masks, const int* __restrict__ row_ptr, int* __restrict__ col_idx,
+                  uint16_t* __restrict__ vals) {
+  const int br = blockIdx.x, lane = threadIdx.x & 31;
+  const int gi = blockIdx.y * kFillWarps + (threadIdx.x >> 5);
+  if (gi >= ngroups) return;
+  // the masks of the row up to this group, 32 at a time, and the row's first
+  // output block load together: what follows waits for one latency
+  const uint32_t* row = masks + (long long)br * ngroups;
+  const int first = __ldg(row_ptr + br);
+  uint32_t mask = 0;
+  int before = 0;
+  for (int g0 = 0; g0 <= gi; g0 += 32) {
+    const uint32_t w = g0 + lane <= gi ? __ldg(row + g0 + lane) : 0u;
+    if (g0 + lane < gi) before += __popc(w);
+    mask = __shfl_sync(0xffffffffu, w, gi - g0 < 32 ? gi - g0 : 31);
+  }
+  if (!mask) return;
+  for (int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  const int lpb = bC / 8, gblk = 32 / lpb;
+  const int pieces = bR * lpb / 32;       // 32 x 16 bytes each (bR and lpb are even, bR a multiple of 16)
+  long long pos = (long long)first + before;   // output block of the piece
+  const uint16_t* arow = A + (long long)br * bR * lda;
+  int b = -1, piece = 0;                  // block of the group being copied and its next piece
+  for (;;) {
+    uint4 v[4];
+    long long at[4];
+    int n = 0;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      if (b < 0) {
+        if (!mask) break;
+        b = __ffs(mask) - 1;
+        mask &= mask - 1;
+        if (lane == 0) col_idx[pos] = gi * gblk + b;
+      }
+      const int c = piece * 32 + lane, x = c / lpb, y = c % lpb;
+      v[t] = __ldg(reinterpret_cast<const uint4*>(arow + (long long)x * lda + (long long)(gi * gblk + b) * bC + y * 8));
+      at[t] = pos * (bR * lpb) + c;
+      ++n;
+      if (++piece == pieces) {
+        piece = 0;
+        b = -1;
+        ++pos;
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      if (t < n) reinterpret_cast<uint4*>(vals)[at[t]] = v[t];
+    if (n < 4) return;
+  }
+}
+
+// The same without masks (a caller with no workspace): finds the blocks again,
+// then writes col_idx and copies the kept blocks. One CTA per block row.
+__global__ void __launch_bounds__(kConvThreads)
+    k_fill_rescan(const uint16_t* __restrict__ A, long long lda, int bR, int bC, int KB,
+                  const int* __restrict__ row_ptr, int* __restrict__ col_idx, uint16_t* __restrict__ vals) {
+  extern __shared__ uint32_t sm[];  // masks[ngroups], offsets[ngroups]
+  const int br = blockIdx.x;
+  const int lpb = bC / 8;                 // lanes per block
+  const int gblk = 32 / lpb;              // blocks per warp pass
+  const int ngroups = (KB + gblk - 1) / gblk;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  uint32_t* masks = sm;
+  uint32_t* offs = sm + ngroups;
+  const uint16_t* arow = A + (long long)br * bR * lda;
+  for (int gi = warp; gi < ngroups; gi += nwarps) {
+    const int j = gi * gblk + lane / lpb;   // block column of this lane
+    const int sub = lane % lpb;
+    bool nz = false;
+    if (j < KB) {
+      const uint16_t* p = arow + (long long)j * bC + sub * 8;
+      for (int x0 = 0; x0 < bR && !nz; x0 += 8) {
+        uint4 v[8];
+#pragma unroll
+        for (int x = 0; x < 8; ++x) v[x] = __ldg(reinterpret_cast<const uint4*>(p + (long long)(x0 + x) * lda));
+#pragma unroll
+        for (int x = 0; x < 8; ++x) nz = nz || any_nonzero_h8(v[x]);
+      }
+    }
+    const uint32_t bal = __ballot_sync(0xffffffffu, nz);
+    uint32_t mask = 0;
+    const uint32_t lm = (lpb >= 32) ? 0xffffffffu : ((1u << lpb) - 1u);
+    for (int b = 0; b < gblk; ++b)
+      if ((bal >> (b * lpb)) & lm) mask |= 1u << b;
+    if (lane == 0) masks[gi] = mask;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -108,9 +205,36 @@ __global__ void __launch_bounds__(kConvThreads)
 }
 
 // Exclusive scan of counts[0..n) into row_ptr[0..n] (row_ptr[0] = 0); one CTA.
-__global__ void __launch_bounds__(1024) k_scan_counts(const int* counts, int* row_ptr, int n) {
+// With masks (n rows of ngroups words), a row's count is its set bits, and
+// counts is row_ptr + 1, where they are kept between the two passes.
+// total (may be NULL): host-visible memory that gets row_ptr[n].
+__global__ void __launch_bounds__(1024)
+    k_scan_counts(const int* counts, int* row_ptr, int n, const uint32_t* masks, int ngroups, int* total) {
   __shared__ long long warp_sums[32];
+  grid_dep_launch_dependents();
+  grid_dep_wait();
   const int t = threadIdx.x, T = blockDim.x;
+  if (masks) {
+    // a warp a row, several rows' words in flight
+    const int lane = t & 31;
+    for (long long r0 = t >> 5; r0 < n; r0 += 8 * (T >> 5)) {
+      int c[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const long long r = r0 + u * (T >> 5);
+        c[u] = r < n && lane < ngroups ? __popc(__ldg(masks + r * ngroups + lane)) : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const long long r = r0 + u * (T >> 5);
+        if (r < n)
+          for (int g = 32 + lane; g < ngroups; g += 32) c[u] += __popc(__ldg(masks + r * ngroups + g));
+        c[u] = __reduce_add_sync(0xffffffffu, c[u]);
+        if (lane == 0 && r < n) row_ptr[r + 1] = c[u];
+      }
+    }
+    __syncthreads();
+  }
   const long long per = (n + T - 1) / T;
   const long long lo = min((long long)n, t * per), hi = min((long long)n, lo + per);
   long long s = 0;
@@ -138,6 +262,7 @@ __global__ void __launch_bounds__(1024) k_scan_counts(const int* counts, int* ro
     run += counts[i];
     row_ptr[i + 1] = (int)run;
   }
+  if (total && (n ? hi == n && lo < hi : t == 0)) *total = (int)run;
 }
 
 // Structure checks. bad[0] |= 1: row_ptr[0] != 0 or not monotone or
@@ -301,8 +426,7 @@ unsigned grid_for(size_t n) {
 }  // namespace
 
 spmm_status scan_counts(const int* counts, int* row_ptr, int n, cudaStream_t s) {
-  k_scan_counts<<<1, 1024, 0, s>>>(counts, row_ptr, n);
-  SPMM_CUDA_TRY(cudaGetLastError());
+  SPMM_CUDA_TRY(launch_kernel(&k_scan_counts, dim3(1), dim3(1024), 0, s, counts, row_ptr, n, (const uint32_t*)nullptr, 0, (int*)nullptr));
   return SPMM_OK;
 }
 
@@ -327,48 +451,92 @@ static spmm_status conv_checks(const void* A, int M, int K, int lda, int bR, int
   return SPMM_OK;
 }
 
-spmm_status spmm_dense_to_bcsr_count(const void* A, int M, int K, int lda, int bR, int bC,
-                                     int* row_ptr, long long* nnzb_out, void* stream) {
-  spmm_status st = conv_checks(A, M, K, lda, bR, bC);
-  if (st != SPMM_OK) return st;
-  if (!row_ptr || !nnzb_out) return fail(SPMM_ERR_INVALID_ARG, "null pointer");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int MB = M / bR, KB = K / bC;
-  const int gblk = 32 / (bC / 8), ngroups = (KB + gblk - 1) / gblk;
-  // counts go to row_ptr[1..MB] first, then the scan rewrites row_ptr in place
-  // from a copy held in the tail of the same launch sequence.
+// The calling thread's word of pinned memory that a scan writes its total to:
+// a copy into pageable memory would go through a staging buffer of the driver.
+static int* host_total() {
+  struct Word {
+    int* p = nullptr;
+    ~Word() {
+      if (p) cudaFreeHost(p);
+    }
+  };
+  static thread_local Word w;
+  if (!w.p && cudaHostAlloc(reinterpret_cast<void**>(&w.p), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
+    w.p = nullptr;
+  return w.p;
+}
+
+static int mask_groups(int K, int bC) {
+  const int KB = K / bC, gblk = 32 / (bC / 8);
+  return (KB + gblk - 1) / gblk;
+}
+
+// Row counts (and masks, if not NULL), their scan into row_ptr, and the total on the host.
+static spmm_status count_blocks(const void* A, int M, int K, int lda, int bR, int bC, uint32_t* masks, int* row_ptr,
+                                long long* nnzb_out, cudaStream_t s) {
+  const int MB = M / bR, KB = K / bC, ngroups = mask_groups(K, bC);
+  int* total = host_total();
+  if (!total) return fail(SPMM_ERR_CUDA, "no pinned memory for the block count");
+  // counts go to row_ptr[1..MB] first and the scan rewrites row_ptr in place:
+  // each thread reads a count before it writes that slot, and the threads'
+  // slots are disjoint
   int* counts = row_ptr + 1;
   if (MB > 0 && KB > 0) {
-    k_dense_to_bcsr<false><<<MB, kConvThreads, (size_t)ngroups * 8, s>>>(
-        static_cast<const uint16_t*>(A), lda, bR, bC, KB, counts, nullptr, nullptr, nullptr);
-    SPMM_CUDA_TRY(cudaGetLastError());
+    const int warps = std::min(ngroups, masks ? 8 : 32);
+    const unsigned runs = masks ? (unsigned)((ngroups + warps - 1) / warps) : 1u;
+    SPMM_CUDA_TRY(launch_kernel(&k_block_masks, dim3((unsigned)MB, runs), dim3(32u * (unsigned)warps), 0, s,
+                                static_cast<const uint16_t*>(A), (long long)lda, bR, bC, KB, ngroups, masks,
+                                masks ? (int*)nullptr : counts));
   } else if (MB > 0) {
     SPMM_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * MB, s));
   }
-  // in-place scan: counts live in row_ptr[1..MB]; k_scan_counts reads all
-  // counts of a thread's chunk before writing, and chunks are disjoint and
-  // shifted by one, so read counts[i] then write row_ptr[i+1] = counts[i]'s slot.
-  k_scan_counts<<<1, 1024, 0, s>>>(counts, row_ptr, MB);
-  SPMM_CUDA_TRY(cudaGetLastError());
-  int total = 0;
-  SPMM_CUDA_TRY(cudaMemcpyAsync(&total, row_ptr + MB, sizeof(int), cudaMemcpyDeviceToHost, s));
+  SPMM_CUDA_TRY(launch_kernel(&k_scan_counts, dim3(1), dim3(1024), 0, s, static_cast<const int*>(counts), row_ptr, MB,
+                              static_cast<const uint32_t*>(KB > 0 ? masks : nullptr), ngroups, total));
   SPMM_CUDA_TRY(cudaStreamSynchronize(s));
-  *nnzb_out = total;
+  *nnzb_out = *static_cast<volatile int*>(total);
   return SPMM_OK;
+}
+
+spmm_status spmm_dense_to_bcsr_count(const void* A, int M, int K, int lda, int bR, int bC,
+                                     int* row_ptr, long long* nnzb_out, void* stream) {
+  return spmm_dense_to_bcsr_count_masks(A, M, K, lda, bR, bC, row_ptr, nullptr, nnzb_out, stream);
+}
+
+long long spmm_dense_to_bcsr_mask_words(int M, int K, int bR, int bC) {
+  if (M < 0 || K < 0 || bR < 16 || bC < 16 || bR % 16 || bC % 16 || bC > 256) return -1;
+  return (long long)(M / bR) * mask_groups(K, bC);
+}
+
+spmm_status spmm_dense_to_bcsr_count_masks(const void* A, int M, int K, int lda, int bR, int bC, int* row_ptr,
+                                           unsigned* masks, long long* nnzb_out, void* stream) {
+  spmm_status st = conv_checks(A, M, K, lda, bR, bC);
+  if (st != SPMM_OK) return st;
+  if (!row_ptr || !nnzb_out) return fail(SPMM_ERR_INVALID_ARG, "null pointer");
+  return count_blocks(A, M, K, lda, bR, bC, masks, row_ptr, nnzb_out, static_cast<cudaStream_t>(stream));
 }
 
 spmm_status spmm_dense_to_bcsr_fill(const void* A, int M, int K, int lda, int bR, int bC,
                                     const int* row_ptr, int* col_idx, void* vals, void* stream) {
+  return spmm_dense_to_bcsr_fill_masks(A, M, K, lda, bR, bC, row_ptr, nullptr, col_idx, vals, stream);
+}
+
+spmm_status spmm_dense_to_bcsr_fill_masks(const void* A, int M, int K, int lda, int bR, int bC, const int* row_ptr,
+                                          const unsigned* masks, int* col_idx, void* vals, void* stream) {
   spmm_status st = conv_checks(A, M, K, lda, bR, bC);
   if (st != SPMM_OK) return st;
   const int MB = M / bR, KB = K / bC;
   if (MB == 0 || KB == 0) return SPMM_OK;
   if (!row_ptr || !col_idx || !vals) return fail(SPMM_ERR_INVALID_ARG, "null pointer");
   if (reinterpret_cast<uintptr_t>(vals) & 15) return fail(SPMM_ERR_MISALIGNED, "vals must be 16-byte aligned");
-  const int gblk = 32 / (bC / 8), ngroups = (KB + gblk - 1) / gblk;
-  k_dense_to_bcsr<true><<<MB, kConvThreads, (size_t)ngroups * 8, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint16_t*>(A), lda, bR, bC, KB, nullptr, row_ptr, col_idx,
-      static_cast<uint16_t*>(vals));
+  const int ngroups = mask_groups(K, bC);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const uint16_t* a = static_cast<const uint16_t*>(A);
+  if (masks)
+    k_fill_masked<<<dim3((unsigned)MB, (unsigned)((ngroups + kFillWarps - 1) / kFillWarps)), 32 * kFillWarps, 0, s>>>(
+        a, lda, bR, bC, ngroups, masks, row_ptr, col_idx, static_cast<uint16_t*>(vals));
+  else
+    k_fill_rescan<<<MB, kConvThreads, (size_t)ngroups * 8, s>>>(a, lda, bR, bC, KB, row_ptr, col_idx,
+                                                               static_cast<uint16_t*>(vals));
   SPMM_CUDA_TRY(cudaGetLastError());
   return SPMM_OK;
 }
