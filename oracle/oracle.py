@@ -34,7 +34,7 @@ def build(ref_tree=None):
     (ref_tree, else reference_tree()) also the _ref build from its sources."""
     subprocess.run(["make", "-s", "-C", HERE, "liboracle.so"], check=True)
     ref_tree = ref_tree or reference_tree()
-    if ref_tree and os.path.isdir(ref_tree):
+    if ref_tree and os.path.exists(os.path.join(ref_tree, "Matrix.cu")):   # not where its folder is empty
         subprocess.run(["make", "-s", "-C", HERE, "ref", "REF=" + ref_tree], check=True)
     if os.path.exists(REF_CUBIN):
         subprocess.run(["make", "-s", "-C", HERE, "libref_wmma.so"], check=True)
