@@ -51,7 +51,8 @@ typedef struct spmm_config {
   int stages;    /* pipeline depth 2..8 (0 = auto)                                   */
   int ctas_per_sm; /* persistent grid = SMs x this (0 = auto)                          */
   int acc_buffers; /* tcgen05: TMEM accumulators per CTA, 1 or 2 (0 = auto)          */
-  int schedule;    /* tcgen05: 0 = static item stride, 1 = atomic work queue,
+  int schedule;    /* tcgen05: 0 = static item stride, 1 = dynamic (a CTA takes
+                      over blocks of its grid that have not started),
                       2 = per-matrix plan (a tuner-table mark: spmm_bcsr_plan_create
                       builds the plan, whose runs chain with
                       SPMM_RUN_INPUTS_READY; spmm_bcsr_mm runs it as 1)       */
@@ -101,6 +102,11 @@ const char* spmm_last_error(void);
  */
 spmm_status spmm_bcsr_mm(const spmm_bcsr_desc* A, const spmm_dense_desc* B, int N,
                          float* C, int ldc, const spmm_config* cfg, void* stream);
+/* The same with the number of stored blocks (row_ptr's last entry), which the
+ * host often knows and the library would have to copy from the device: only the
+ * choice of kernel depends on it, when cfg gives none. Negative: not known. */
+spmm_status spmm_bcsr_mm_nnzb(const spmm_bcsr_desc* A, long long nnzb, const spmm_dense_desc* B, int N,
+                              float* C, int ldc, const spmm_config* cfg, void* stream);
 
 /* Checks row_ptr / col_idx on the device (monotone, row_ptr[0] == 0,
  * row_ptr[M/bR] == nnzb, col_idx in [0, K/16), strictly ascending within a
@@ -337,13 +343,14 @@ spmm_status spmm_dense_mm(const void* A, int lda, const spmm_dense_desc* B, int 
  * No counterpart in the reference (its harness sweeps kernels by hand).
  * The configuration space: a fixed table of spmm_tune_config_count() entries
  * (41: five mma.sync column tiles and depths; tcgen05 column tiles, depths,
- * accumulator counts, static or work-queue schedules and split-K; the 64-row
+ * accumulator counts, static or dynamic schedules and split-K; the 64-row
  * tcgen05 pipeline's column tiles and schedules). Not every entry has a kernel
  * for every block height and type. */
 int spmm_tune_config_count(void);
 spmm_status spmm_tune_config(int i, spmm_config* out);
 /* The configuration spmm_bcsr_mm runs when given none (the library's fixed
- * heuristic), as a table entry. */
+ * heuristic), as a table entry: its choice where the number of rows and of
+ * stored blocks does not tip it (see spmm_bcsr_mm_nnzb). */
 spmm_status spmm_default_config(int bR, spmm_dtype dtype, int N, spmm_config* out);
 /* SPMM_OK if `cfg` has a kernel for (bR, dtype, N), else SPMM_ERR_UNSUPPORTED. */
 spmm_status spmm_config_supported(int bR, spmm_dtype dtype, int N, const spmm_config* cfg);
@@ -476,15 +483,14 @@ spmm_status spmm_bcsr_plan_destroy(spmm_bcsr_plan* plan);
  * host application or allocator that owns all device memory, a memory budget
  * that forbids the CUDA allocator, code that must not allocate while a stream
  * is being captured): the same product as spmm_bcsr_mm on the tcgen05 pipeline
- * with its work queue, but its scratch -- the device error word and the
- * queue's two counters, 12 bytes -- lives in a fixed 256-byte __device__ array
- * compiled into the library (held on every GPU that loads the library until
- * the process exits), and the call allocates nothing. The caller still passes
+ * with its dynamic schedule, but its scratch -- the device error word -- lives
+ * in a fixed 256-byte __device__ array compiled into the library (held on every
+ * GPU that loads the library until the process exits), and the call allocates
+ * nothing. The caller still passes
  * A, B and C.
  *  - fp16, bf16 and split fp16 only (E4M3 runs on a path with allocated scratch).
  *  - Fewer than 2^30 work items (block rows x column tiles of the tile that
- *    runs x split-K slices): the queue counters are 32-bit. Larger problems
- *    return SPMM_ERR_SCRATCH_TOO_SMALL.
+ *    runs x split-K slices). Larger problems return SPMM_ERR_SCRATCH_TOO_SMALL.
  *  - K == 0 zeroes the C window (cudaMemset2DAsync, which allocates nothing).
  *  - The first call on each device looks up the array's device address
  *    (cudaGetSymbolAddress) and keeps it for the life of the process; make that

@@ -70,6 +70,8 @@ _SIGS = {
     "spmm_device_error_check": (c_int, [c_vp]),
     "spmm_bcsr_mm": (c_int, [ctypes.POINTER(BcsrDesc), ctypes.POINTER(DenseDesc), c_int, c_vp,
                              c_int, ctypes.POINTER(Config), c_vp]),
+    "spmm_bcsr_mm_nnzb": (c_int, [ctypes.POINTER(BcsrDesc), c_ll, ctypes.POINTER(DenseDesc), c_int, c_vp, c_int,
+                                  ctypes.POINTER(Config), c_vp]),
     "spmm_bcsr_validate": (c_int, [c_vp, c_vp, c_int, c_int, c_int, c_ll, c_vp]),
     "spmm_gpu_gen_structure": (c_int, [c_int, c_int, c_int, c_int, c_double, c_double, c_ull, c_vp, c_vp, c_ll,
                                        ctypes.POINTER(c_ll), c_vp]),

@@ -17,6 +17,10 @@ def _torch():
     return torch
 
 
+def _addr(t):
+    return None if t is None else t.data_ptr()
+
+
 def _ptr(t):
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
@@ -92,10 +96,8 @@ def spmm(A: BCSR, B, N=None, C=None, cfg: Optional[Config] = None, stream=None, 
     ldc = int(C.stride(0)) if ldc is None else int(ldc)
     a = A.desc()
     b = _dense_desc(B, B_lo, b_scale, ldb=B.stride(0))
-    st = lib().spmm_bcsr_mm(ctypes.byref(a), ctypes.byref(b), N, ctypes.c_void_p(C.data_ptr()),
-                            ldc, ctypes.byref(cfg) if cfg is not None else None,
-                            stream_handle(stream))
-    check(st)
+    check(lib().spmm_bcsr_mm_nnzb(ctypes.byref(a), A.nnzb, ctypes.byref(b), N, ctypes.c_void_p(C.data_ptr()), ldc,
+                                  ctypes.byref(cfg) if cfg is not None else None, stream_handle(stream)))
     return C
 
 
@@ -267,39 +269,42 @@ def csr_mm(row_ptr, col_idx, vals, K, B, N=None, C=None, stream=None, ldc=None):
     return C
 
 
-def _ref_launch(fn, hdr, idx, data, B, C, M, N, K, stream, extra=()):
-    st = fn(_ptr(hdr), _ptr(idx), _ptr(data), _ptr(B), _ptr(C), int(M), int(N), *extra, int(K),
-            stream_handle(stream))
-    check(st)
+def _ref_launch(bR, hdr, idx, data, B, C, M, N, K, stream):
+    """The reference-shaped call: contiguous fp16 operands given by their arrays
+    (what the library's <name>_launch entries do, with the stored blocks known)."""
+    a = BcsrDesc()
+    a.M, a.K, a.bR, a.bC = int(M), int(K), bR, 16
+    a.row_ptr, a.col_idx, a.vals = _addr(hdr), _addr(idx), _addr(data)
+    b = DenseDesc()
+    b.data, b.scale, b.ldb = _addr(B), 1.0, int(N)
+    check(lib().spmm_bcsr_mm_nnzb(ctypes.byref(a), -1 if idx is None else idx.numel(), ctypes.byref(b), int(N),
+                                  _ptr(C), int(N), None, stream_handle(stream)))
     return C
 
 
 # Reference-shaped launchers (src/cuda_kernels.cuh:39-114 argument order, + K, + stream).
 def sparseMatrixMulTensor(hdr, idx, data, B, C, M, N, K, stream=None):
-    return _ref_launch(lib().sparseMatrixMulTensor_launch, hdr, idx, data, B, C, M, N, K, stream)
+    return _ref_launch(16, hdr, idx, data, B, C, M, N, K, stream)
 
 
 def sparseMatrixMulTensor32x16(hdr, idx, data, B, C, M, N, K, stream=None):
-    return _ref_launch(lib().sparseMatrixMulTensor32x16_launch, hdr, idx, data, B, C, M, N, K, stream)
+    return _ref_launch(32, hdr, idx, data, B, C, M, N, K, stream)
 
 
 def sparseMatrixMulTensor64x16(hdr, idx, data, B, C, M, N, K, stream=None):
-    return _ref_launch(lib().sparseMatrixMulTensor64x16_launch, hdr, idx, data, B, C, M, N, K, stream)
+    return _ref_launch(64, hdr, idx, data, B, C, M, N, K, stream)
 
 
 def sparseMatrixMulTensorAdaptive(hdr, idx, data, B, C, M, N, colBlocksPerRow, K, stream=None):
-    return _ref_launch(lib().sparseMatrixMulTensorAdaptive_launch, hdr, idx, data, B, C, M, N, K,
-                       stream, (int(colBlocksPerRow),))
+    return _ref_launch(16, hdr, idx, data, B, C, M, N, K, stream)
 
 
 def sparseMatrixMulTensorAdaptive32x16(hdr, idx, data, B, C, M, N, colBlocksPerRow, K, stream=None):
-    return _ref_launch(lib().sparseMatrixMulTensorAdaptive32x16_launch, hdr, idx, data, B, C, M, N,
-                       K, stream, (int(colBlocksPerRow),))
+    return _ref_launch(32, hdr, idx, data, B, C, M, N, K, stream)
 
 
 def sparseMatrixMulTensorAdaptive64x16(hdr, idx, data, B, C, M, N, colBlocksPerRow, K, stream=None):
-    return _ref_launch(lib().sparseMatrixMulTensorAdaptive64x16_launch, hdr, idx, data, B, C, M, N,
-                       K, stream, (int(colBlocksPerRow),))
+    return _ref_launch(64, hdr, idx, data, B, C, M, N, K, stream)
 
 
 def dense_to_bcsr(A_half, bR=16, bC=16, stream=None):

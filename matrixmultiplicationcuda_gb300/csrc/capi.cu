@@ -124,26 +124,6 @@ unsigned* device_error_word() {
   return g_err_word[d];
 }
 
-namespace {
-constexpr int kQueueSlots = 256;
-unsigned* g_queue_pool[kMaxDevices] = {nullptr};
-unsigned g_queue_next[kMaxDevices] = {0};
-}  // namespace
-
-unsigned* work_queue_slot() {
-  int d = current_device();
-  if (d < 0 || d >= kMaxDevices) return nullptr;
-  std::lock_guard<std::mutex> lk(g_mu);
-  if (!g_queue_pool[d]) {
-    void* p = nullptr;
-    if (cudaMalloc(&p, kQueueSlots * 2 * sizeof(unsigned)) != cudaSuccess) return nullptr;
-    if (cudaMemset(p, 0, kQueueSlots * 2 * sizeof(unsigned)) != cudaSuccess) return nullptr;
-    g_queue_pool[d] = static_cast<unsigned*>(p);
-  }
-  const unsigned i = g_queue_next[d]++ % kQueueSlots;
-  return g_queue_pool[d] + 2 * i;
-}
-
 unsigned long long wait_limit_ns() {
   static unsigned long long v = [] {
     const char* s = std::getenv("SPMM_WAIT_LIMIT_NS");
@@ -297,7 +277,76 @@ spmm_status spmm_device_error_check(void* stream) {
   return SPMM_OK;
 }
 
-spmm_status spmm_bcsr_mm(const spmm_bcsr_desc* A, const spmm_dense_desc* B, int N, float* C,
+}  // extern "C"
+
+namespace spmm {
+
+// What a product with no configuration runs, from its sizes and (nnzb >= 0) the
+// number of stored blocks. Times in us on one GB300, back to back, fp16, the
+// line's two sides:
+//   64-row blocks: tc512 (two accumulators) from 1024 columns and 256 tiles on
+//     (8192^2, 20 %, N 1024: 41.8 against 48.6 for the 64-row pipeline and 48.9
+//     for tc256; at half as many tiles 11.4 against 12.0, with log-normal rows
+//     35 against 31); else the 64-row pipeline (8192^2, 8 %, N 128: 9.7 against
+//     11.5 for tc128; log-normal, N 512: 47 against 62 for tc256), but tc256
+//     where rows are known to be short (1 %, N 512: 7.8 against 8.5) and
+//     mma.sync where there is next to nothing to do (1024^2, 8 %: 3.8 against
+//     5.6).
+//   32- and 16-row blocks: mma.sync, whose CTAs are small, unless rows are known
+//     to be long, where a tcgen05 CTA's deeper ring pays: 32 rows, 8192^2, 8 %
+//     (41 blocks a row), N 512: 18.2 against 28.8; 1 % (5 a row): 8.8 against
+//     8.5. 16 rows, 8 %: 26.5 against 30.4; 1 %: 11.5 against 9.2; 8192^2 with
+//     log-normal rows, 8 %: 51 against 123. Its column tile is 256 wide, so
+//     narrower products stay.
+//   split fp16, 64-row blocks above 128 columns: the 64-row pipeline (16384^2,
+//     2 %, N 512: 30.5 against 33.9 for tc256).
+//   e4m3: mma.sync, which takes any block scale.
+spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnzb) {
+  spmm_config c;
+  std::memset(&c, 0, sizeof(c));
+  const double row = nnzb >= 0 && M > 0 ? (double)nnzb * bR / M : -1.0;   // blocks per block row
+  auto tc = [&](int kernel, int nt, int acc) {
+    c.kernel = kernel;
+    c.n_tile = nt;
+    c.acc_buffers = acc;
+    c.schedule = 1;
+    c.split_k = 1;
+  };
+  if (dtype != SPMM_E4M3) {
+    if (bR == 64 && dtype == SPMM_F16_SPLIT) {
+      if (N <= 128)
+        tc(2, 128, 2);
+      else
+        tc(3, 256, 0);
+    } else if (bR == 64) {
+      const bool tiles512 = N >= 1024 && (N % 512 == 0 || N % 512 > 256) && (long long)(M / 64) * ((N + 511) / 512) >= 256;
+      if (tiles512)
+        tc(2, 512, 2);
+      else if (row >= 0 && nnzb > 100 && row < 8 && N > 128)
+        tc(2, 256, 2);
+      else if (nnzb < 0 || nnzb > 100)
+        tc(3, 256, 0);
+    } else if (dtype != SPMM_F16_SPLIT && N > 128 && row >= (bR == 16 ? 16 : 12)) {
+      tc(2, 256, 2);
+    }
+    if (c.kernel != 0) return c;
+  }
+  c.kernel = 1;
+  c.n_tile = bR == 64 && dtype != SPMM_E4M3 && dtype != SPMM_F16_SPLIT ? 64 : mma_default_nt(bR, dtype, N);
+  c.stages = 4;
+  return c;
+}
+
+}  // namespace spmm
+
+extern "C" {
+
+spmm_status spmm_bcsr_mm(const spmm_bcsr_desc* A, const spmm_dense_desc* B, int N, float* C, int ldc,
+                         const spmm_config* cfg, void* stream) {
+  return spmm_bcsr_mm_nnzb(A, -1, B, N, C, ldc, cfg, stream);
+}
+
+spmm_status spmm_bcsr_mm_nnzb(const spmm_bcsr_desc* A, long long nnzb, const spmm_dense_desc* B, int N, float* C,
                          int ldc, const spmm_config* cfg, void* stream) {
   g_last_error.clear();
   if (!A || !B) return fail(SPMM_ERR_INVALID_ARG, "null descriptor");
@@ -337,14 +386,25 @@ spmm_status spmm_bcsr_mm(const spmm_bcsr_desc* A, const spmm_dense_desc* B, int 
   std::memset(&r.cfg, 0, sizeof(r.cfg));
   if (cfg) r.cfg = *cfg;
   r.stream = static_cast<cudaStream_t>(stream);
-  if (r.cfg.kernel == 3) return launch_tc64(r);
-  // kernel 0: tcgen05 for 64-row blocks (not e4m3, whose tcgen05 kernels need
-  // power-of-two block scales), mma.sync otherwise
-  if (r.cfg.kernel == 2 || (r.cfg.kernel == 0 && A->bR == 64 && !e4m3)) {
-    spmm_status st = launch_tc(r);
-    if (st != SPMM_ERR_UNSUPPORTED || r.cfg.kernel == 2) return st;
+  if (r.cfg.kernel == 0) {
+    // a configuration without a kernel may still set parts of one
+    const spmm_config want = r.cfg;
+    const bool plain = want.n_tile == 0 && want.stages == 0 && want.ctas_per_sm == 0 && want.acc_buffers == 0 &&
+                       want.schedule == 0 && want.split_k <= 1;
+    if (plain) {
+      r.cfg = default_config(A->bR, A->dtype, A->M, N, nnzb);
+    } else {
+      r.cfg.kernel = A->bR == 64 && !e4m3 ? 2 : 1;
+    }
+    spmm_status st = r.cfg.kernel == 1 ? launch_mma(r) : r.cfg.kernel == 3 ? launch_tc64(r) : launch_tc(r);
+    if (st != SPMM_ERR_UNSUPPORTED || r.cfg.kernel == 1) return st;
     g_last_error.clear();
+    r.cfg = want;
+    r.cfg.kernel = 0;
+    return launch_mma(r);
   }
+  if (r.cfg.kernel == 3) return launch_tc64(r);
+  if (r.cfg.kernel == 2) return launch_tc(r);
   return launch_mma(r);
 }
 
@@ -357,7 +417,10 @@ spmm_status spmm_hcsr_mm(const spmm_bcsr_desc* A, const spmm_csr_desc* R, const 
   if (A->M > 0 && !R->row_ptr) return fail(SPMM_ERR_INVALID_ARG, "null CSR row_ptr");
   spmm_config c;
   std::memset(&c, 0, sizeof(c));
-  if (cfg) c = *cfg;
+  if (cfg)
+    c = *cfg;
+  else
+    c.schedule = 1;   // the grid's pending blocks as items
   if (c.kernel != 0 && c.kernel != 2) return fail(SPMM_ERR_UNSUPPORTED, "the hybrid product runs on kernel 2");
   if (c.split_k > 1) return fail(SPMM_ERR_UNSUPPORTED, "the hybrid product has no split-K");
   c.kernel = 2;

@@ -187,7 +187,10 @@ extern "C" spmm_status spmm_hcsr_plan_run(const spmm_hcsr_plan* p, const spmm_de
   if (!p || !B) return fail(SPMM_ERR_INVALID_ARG, "null plan or descriptor");
   spmm_config c;
   std::memset(&c, 0, sizeof(c));
-  if (cfg) c = *cfg;
+  if (cfg)
+    c = *cfg;
+  else
+    c.schedule = 1;   // the grid's pending blocks as items
   if (c.kernel != 0 && c.kernel != 2) return fail(SPMM_ERR_UNSUPPORTED, "the planned hybrid product runs on kernel 2");
   c.kernel = 2;
   if (N < 0) return fail(SPMM_ERR_INVALID_ARG, "negative size");

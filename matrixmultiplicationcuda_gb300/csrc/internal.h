@@ -46,11 +46,6 @@ cudaError_t launch_kernel(void (*fn)(KArgs...), dim3 grid, dim3 block, size_t sm
   return cudaLaunchKernelEx(&cfg, fn, static_cast<Args&&>(args)...);
 }
 unsigned* device_error_word();                   // per-device error word (lazy)
-// A zeroed pair {next item, CTAs done} for one persistent launch's work queue.
-// Slots rotate over a per-device pool; each launch's last CTA zeroes its slot
-// again, so a slot is reusable as soon as the launch that used it has ended.
-unsigned* work_queue_slot();
-
 // cuTensorMapEncodeTiled through the runtime's driver entry point.
 spmm_status encode_tile_map_2d(CUtensorMap* map, CUtensorMapDataType dt, const void* base,
                                uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
@@ -73,10 +68,8 @@ struct LaunchRequest {
   long long ldc;
   spmm_config cfg;
   cudaStream_t stream;
-  // Caller-provided scratch (both NULL for every entry point except the
-  // allocation-free one): the device error word and the work-queue pair.
+  // caller-provided device error word (the allocation-free entry point's)
   unsigned* err_word = nullptr;
-  unsigned* queue = nullptr;
   // hybrid product: the CSR part added by the tcgen05 pipeline's epilogue
   const spmm_csr_desc* csr = nullptr;
   // planned hybrid product: A holds gather blocks (col_idx = -(g + 1)) whose
@@ -90,6 +83,7 @@ struct LaunchRequest {
   const int* pair = nullptr;
   const int* parts = nullptr;
   unsigned* counters = nullptr;
+  unsigned* queue = nullptr;   // the plan's work queue {next item, CTAs done}
   int plan_items = 0;
   // no kernel launched on the stream since its last host synchronisation
   // writes A or B: the pipeline's copies and MMAs may start before the
@@ -117,7 +111,9 @@ spmm_status launch_tc64(const LaunchRequest& r);
 bool mma_supported(int bR, spmm_dtype dtype, int N, const spmm_config& cfg);
 bool tc_supported(int bR, spmm_dtype dtype, int N, const spmm_config& cfg);
 bool tc64_supported(int bR, spmm_dtype dtype, int N, const spmm_config& cfg);
-int mma_default_nt(int bR, spmm_dtype dtype, int N);   // the column tile spmm_bcsr_mm picks by default
+int mma_default_nt(int bR, spmm_dtype dtype, int N);   // the mma.sync pipeline's default column tile
+// What spmm_bcsr_mm runs with no configuration (nnzb < 0: not known).
+spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnzb);
 
 unsigned long long wait_limit_ns();              // bounded-wait limit for device waits
 

@@ -4,9 +4,9 @@
 // allocator or a memory budget that forbids the CUDA allocator, plugins whose
 // host application owns every device allocation, and code that must not
 // allocate while a stream is being captured into a CUDA graph. The regular
-// entry point allocates two small device buffers on first use (the device
-// error word and the pool of work-queue counters); this variant takes its
-// scratch from a fixed array compiled into the library instead.
+// entry point allocates a small device buffer on first use (the device error
+// word); this variant takes it from a fixed array compiled into the library
+// instead.
 //
 // The array below is that scratch. It is a file-scope __device__ array, so
 // every GPU that loads the library holds it until the process exits. Host code
@@ -23,7 +23,6 @@ namespace spmm {
 namespace {
 
 // Word 0: device error word (set by a bounded wait that gave up).
-// Words 1-2: the work queue's {next item, CTAs done} pair.
 // The rest pads the array to its alignment.
 constexpr int kScratchWords = 64;
 static __device__ __align__(256) unsigned g_noalloc_scratch[kScratchWords];
@@ -90,9 +89,8 @@ spmm_status spmm_bcsr_mm_noalloc(const spmm_bcsr_desc* A, const spmm_dense_desc*
   run_cfg.kernel = 2;
   run_cfg.schedule = 1;
   // The work items the launch will hold: block rows x column tiles of the
-  // tile that runs x split-K slices. The queue counters are 32-bit and
-  // overshoot the item count by up to the grid size, so a launch may hold
-  // fewer than 2^30 items (the pipeline's own limit).
+  // tile that runs x split-K slices; a launch may hold fewer than 2^30 (the
+  // pipeline's own limit).
   int nt = 0, per_sm = 0;
   if (!tc_geometry(A->bR, A->dtype, N, run_cfg, &nt, &per_sm))
     return fail(SPMM_ERR_UNSUPPORTED, "no tcgen05 kernel for this block height, type and configuration");
@@ -101,13 +99,13 @@ spmm_status spmm_bcsr_mm_noalloc(const spmm_bcsr_desc* A, const spmm_dense_desc*
   if (items >= (1ll << 30))
     return fail(SPMM_ERR_SCRATCH_TOO_SMALL,
                 "problem has " + std::to_string(items) +
-                    " work items; the allocation-free variant's 32-bit queue holds fewer than 2^30");
+                    " work items; the allocation-free variant holds fewer than 2^30");
 
   unsigned* scratch = nullptr;
   spmm_status st = scratch_for_current_device(&scratch);
   if (st != SPMM_OK) return st;
-  // Every call shares the array: the error word and the queue pair start at zero.
-  SPMM_CUDA_TRY(cudaMemsetAsync(scratch, 0, 3 * sizeof(unsigned), s));
+  // Every call shares the array: the error word starts at zero.
+  SPMM_CUDA_TRY(cudaMemsetAsync(scratch, 0, sizeof(unsigned), s));
 
   LaunchRequest r;
   r.A = A;
@@ -118,7 +116,6 @@ spmm_status spmm_bcsr_mm_noalloc(const spmm_bcsr_desc* A, const spmm_dense_desc*
   r.cfg = run_cfg;
   r.stream = s;
   r.err_word = scratch;
-  r.queue = scratch + 1;
   return launch_tc(r);
 }
 

@@ -100,6 +100,40 @@ __device__ __forceinline__ void red_add_f32(float* p, float v) {
   asm volatile("red.global.add.f32 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "f"(v) : "memory");
 }
 
+// Generic-proxy shared-memory writes made visible to the async proxy (TMA,
+// tcgen05.mma / tcgen05.cp operand reads).
+__device__ __forceinline__ void fence_proxy_async_smem() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+// ---- cluster launch control ------------------------------------------------------
+// A persistent CTA takes over a block of its own grid that has not started yet:
+// the grid has one block per work item, the hardware hands pending blocks either
+// to a free SM or to a running CTA that asks, and no counter in global memory is
+// shared by launches, streams or graph replays. The 16-byte answer lands in
+// shared memory through an mbarrier (expect 16 bytes before the request). After
+// an answer of "none left" no further request may be made.
+__device__ __forceinline__ void clc_request(uint32_t answer, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   answer),
+               "r"(bar)
+               : "memory");
+}
+// The block's index in x, or -1: no pending block.
+__device__ __forceinline__ int clc_block(uint32_t answer) {
+  int x;
+  asm volatile(
+      "{\n\t.reg .b128 r;\n\t.reg .pred p;\n\t"
+      "ld.shared.b128 r, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "mov.s32 %0, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n\t}"
+      : "=r"(x)
+      : "r"(answer)
+      : "memory");
+  return x;
+}
+
 // ---- cp.async (4 or 16 bytes per thread, global -> shared) ------------------------
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");

@@ -18,8 +18,9 @@
 //     in the K-major canonical layout (8-row groups 256 B apart); the blocks
 //     of a group are contiguous in memory and arrive in one copy.
 //
-// Warp roles (11 warps, two CTAs per SM): warp 0 takes items (static stride,
-// or from a work queue a few groups before the current item is copied),
+// Warp roles (11 warps, two CTAs per SM): warp 0 takes items (its own block's,
+// then the grid's pending blocks, a static stride, or a plan's work queue; the
+// next one is claimed a few groups before the current item is copied),
 // publishes them through an item ring and copies A groups;
 // warps 2, 3, 8, 9 copy the B panels (a TMA instruction holds its issuing
 // thread for ~200 ns, so four threads share them); warp 1 (one thread) issues
@@ -58,8 +59,9 @@ struct TcParams {
   unsigned long long timeout_ns;
   unsigned* err;
   int panel3d;      // B panel loaded by one 3-D copy (N % 64 == 0)
-  unsigned* queue;  // [0] next item, [1] CTAs done; NULL = static item striding
-  int claim_ahead;  // work queue: claim the next item when this many groups of the current one are left to copy
+  int dynamic;      // later items: 1 = the grid's pending blocks (one block per item), 0 = the queue or a static stride
+  unsigned* queue;  // a plan's queue: [0] next item, [1] CTAs done; NULL = none
+  int claim_ahead;  // dynamic, queue: claim the next item when this many groups of the current one are left to copy
   int inputs_ready; // no kernel earlier on the stream writes A or B (see the dependency wait below)
   int split;        // items per (block row, column tile); > 1: partial sums added into C
   // hybrid (BCSR + CSR): the CSR part's entries are added in the epilogue
@@ -213,6 +215,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 5 + 2 * kQ);
   int* s_item = reinterpret_cast<int*>(tmem_slot + 1);      // kQ x {item, start, end, column tile}
   int* s_role = s_item + 4 * kQ;                            // a split row's role, set by the epilogue
+  // claims of pending blocks: the 16-byte answer and its barrier, 512 bytes into
+  // the 1 KB after the ring (the barriers and the item ring take up to 320)
+  const uint32_t answer = smem_u32(bars) + 512, claim_bar = answer + 16;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 32) {
@@ -227,6 +232,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       mbar_init(tempty0 + 8 * b, 4);
     }
     mbar_init(done_bar, Cfg::kIssuers);
+    mbar_init(claim_bar, 1);
     for (int q = 0; q < kQ; ++q) {
       mbar_init(qfull0 + 8 * q, 1);
       mbar_init(qempty0 + 8 * q, Cfg::kIssuers + kBIssuers + 4);   // MMA issuers, B issuers, epilogue warps
@@ -352,17 +358,47 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         mbar_arrive(qfull0 + 8 * q);
       };
       // Items after the first: static striding (blockIdx.x + k * gridDim.x),
-      // or tickets from the work queue offset by the grid size. A ticket is
-      // taken late, when claim_ahead groups of the current item are left to
-      // copy (< 0: as the item starts), so that a CTA running faster (lighter
-      // items, or an SM it no longer shares) takes more of the items still
-      // unclaimed; its atomic is issued one group before the result is used,
-      // and the item goes into the ring at once. Either way every CTA takes
-      // its items in increasing list order.
-      const bool late = p.queue != nullptr && p.claim_ahead >= 0;
-      auto ticket_item = [&](unsigned t) -> int {
-        const unsigned v = t + gridDim.x;
-        return v < (unsigned)p.n_items ? (int)v : -1;
+      // blocks of the grid that have not started, or tickets from a plan's work
+      // queue offset by the grid size. A claim is made late, when claim_ahead
+      // groups of the current item are left to copy (< 0: as the item starts),
+      // so that a CTA running faster (lighter items, or an SM it no longer
+      // shares) takes more of the items still unclaimed; it is issued one group
+      // before its result is used, and the item goes into the ring at once.
+      // (Claiming two items ahead, with the block ranges and column indices of
+      // the next one loaded early, made short rows no faster and cost every
+      // other shape 5-15 %: the issuing warps' instructions per group count.)
+      // A plan keeps its own queue: its split rows need every CTA to take its
+      // items in list order, which claims of pending blocks do not promise. A
+      // queue that holds nothing beyond the CTAs' first items is not touched:
+      // under the inputs-ready promise a claim waits for the previous kernel,
+      // and the copies of A's last groups would wait with it.
+      const bool no_more = p.queue && (int)gridDim.x >= p.n_items;
+      const bool late = (p.dynamic || p.queue != nullptr) && p.claim_ahead >= 0 && !no_more;
+      uint32_t claims = 0;
+      auto claim = [&]() -> unsigned {
+        if (!p.dynamic) {
+          if (!dep_waited) {
+            grid_dep_wait();
+            dep_waited = true;
+          }
+          return atomicAdd(p.queue, 1u);
+        }
+        fence_proxy_async_smem();   // the last answer has been read
+        mbar_arrive_expect_tx(claim_bar, 16);
+        clc_request(answer, claim_bar);
+        return 0u;
+      };
+      auto claimed_item = [&](unsigned t) -> int {
+        if (!p.dynamic) {
+          const unsigned v = t + gridDim.x;
+          return v < (unsigned)p.n_items ? (int)v : -1;
+        }
+        if (!mbar_wait(claim_bar, claims++ & 1, p.timeout_ns)) {
+          atomicOr(p.err, 4u);
+          failed = true;
+          return -1;
+        }
+        return clc_block(answer);
       };
       int item = (int)blockIdx.x;
       int start = 0, end = 0, tile = 0;
@@ -382,12 +418,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         unsigned ticket = 0;
         if (!late) {
           // the next item's indices load now and are used once this item is copied
-          if (p.queue && !dep_waited) {
-            grid_dep_wait();
-            dep_waited = true;
-          }
-          nitem = p.queue ? ticket_item(atomicAdd(p.queue, 1u))
-                          : (item + (int)gridDim.x < p.n_items ? item + (int)gridDim.x : -1);
+          nitem = no_more ? -1
+                  : p.dynamic || p.queue ? claimed_item(claim())
+                                         : (item + (int)gridDim.x < p.n_items ? item + (int)gridDim.x : -1);
           range(nitem, &nstart, &nend, &ntile);
         }
         const int ngroups = (end - start + G - 1) / G;
@@ -403,16 +436,12 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         for (int j0 = start; j0 < end; j0 += G, ++gs, ++gi) {
           if (late && nitem == -2) {
             if (claimed) {
-              nitem = ticket_item(ticket);
+              nitem = claimed_item(ticket);
               range(nitem, &nstart, &nend, &ntile);
               publish(it + 1, nitem, nstart, nend, ntile);
               if (failed) break;
             } else if (ngroups - gi <= p.claim_ahead + 1) {
-              if (!dep_waited) {
-                grid_dep_wait();
-                dep_waited = true;
-              }
-              ticket = atomicAdd(p.queue, 1u);
+              ticket = claim();
               claimed = true;
             }
           }
@@ -446,17 +475,14 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             }
           }
         }
-        if (failed) break;
+        if (failed) {
+          if (p.dynamic && claimed && nitem == -2) claimed_item(ticket);   // an answer still on its way
+          break;
+        }
         in_ring = late && nitem != -2;
         if (nitem == -2) {   // late claim not made or not used yet (short item)
-          if (!claimed) {
-            if (!dep_waited) {
-              grid_dep_wait();
-              dep_waited = true;
-            }
-            ticket = atomicAdd(p.queue, 1u);
-          }
-          nitem = ticket_item(ticket);
+          if (!claimed) ticket = claim();
+          nitem = claimed_item(ticket);
           range(nitem, &nstart, &nend, &ntile);
         }
         item = nitem;
@@ -465,7 +491,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         tile = ntile;
       }
       // the last CTA to finish resets the queue for the next launch
-      if (p.queue) {
+      if (p.queue && !no_more) {
         if (!dep_waited) grid_dep_wait();
         __threadfence();
         if (atomicAdd(p.queue + 1, 1u) == gridDim.x - 1) {
@@ -1059,8 +1085,6 @@ spmm_status launch_tc(const LaunchRequest& r) {
   p.timeout_ns = wait_limit_ns();
   p.err = r.err_word ? r.err_word : device_error_word();
   p.panel3d = panel3d;
-  // items: static stride by default, or a work queue on request
-  p.queue = r.queue ? r.queue : (r.cfg.schedule >= 1 ? work_queue_slot() : nullptr);
   p.claim_ahead = e->stages - 1;
   p.inputs_ready = r.inputs_ready ? 1 : 0;
   p.csr_row_ptr = r.csr ? r.csr->row_ptr : nullptr;
@@ -1081,7 +1105,7 @@ spmm_status launch_tc(const LaunchRequest& r) {
   p.mbR = stacked ? r.member_bR : 0;
   p.oob_row = (int)rows_bound;
   if (r.items) {
-    if (p.split > 1 || r.csr || r.gather_rows || (p.queue && !r.queue))
+    if (p.split > 1 || r.csr || r.gather_rows)
       return fail(SPMM_ERR_UNSUPPORTED, "a planned product runs without split-K, CSR part or shared work queue");
     p.n_items = r.plan_items;
   }
@@ -1102,14 +1126,19 @@ spmm_status launch_tc(const LaunchRequest& r) {
   int per_sm = std::min(2, std::min(tmem_fit, smem_fit));
   if (r.cfg.ctas_per_sm > 0 && r.cfg.ctas_per_sm < per_sm) per_sm = r.cfg.ctas_per_sm;
   if (per_sm < 1) per_sm = 1;
+  // later items: a plan's queue, or on request the grid's pending blocks (one
+  // block per item; a request for fewer CTAs per SM keeps the static stride,
+  // whose grid it sets)
+  p.queue = r.items ? r.queue : nullptr;
+  p.dynamic = !r.items && r.cfg.schedule >= 1 && r.cfg.ctas_per_sm <= 0 ? 1 : 0;
   long long grid = (long long)sm_count() * per_sm;
-  if (grid > p.n_items) grid = p.n_items;
+  if (grid > p.n_items || p.dynamic) grid = p.n_items;
   if (std::getenv("SPMM_DEBUG"))
     std::fprintf(stderr,
                  "[spmm] tcgen05 bR=%d nt=%d stages=%d acc=%d group=%d smem=%zu tmem=%d per_sm=%d grid=%lld "
-                 "items=%d panel3d=%d queue=%d claim_ahead=%d inputs_ready=%d split=%d\n",
+                 "items=%d panel3d=%d dynamic=%d queue=%d claim_ahead=%d inputs_ready=%d split=%d\n",
                  A.bR, nt, e->stages, e->acc, e->group, e->smem, e->tmem_cols, per_sm, grid, p.n_items, panel3d,
-                 p.queue != nullptr, p.claim_ahead, p.inputs_ready, p.split);
+                 p.dynamic, p.queue != nullptr, p.claim_ahead, p.inputs_ready, p.split);
   SPMM_CUDA_TRY(launch_kernel(e->fn, dim3((unsigned)grid), dim3(kTcThreads), e->smem, r.stream, tmA1, tmAg, tmAlo1,
                               tmAlog, tmB, tmBlo, p));
   return SPMM_OK;

@@ -47,7 +47,7 @@ struct Tc64Params {
   unsigned long long timeout_ns;
   unsigned* err;
   int panel3d;
-  unsigned* queue;
+  int dynamic;      // later items: 1 = the grid's pending blocks (one block per item), 0 = a static stride
 };
 
 // NT: output columns per item (256 or 512); STAGES: ring depth in groups;
@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(kTc64Threads, 1)
   const uint32_t full0 = smem_u32(bars), empty0 = full0 + 8 * STAGES;
   const uint32_t tfull0 = empty0 + 8 * STAGES, tempty0 = tfull0 + 16, done_bar = tempty0 + 16;
   const uint32_t qfull0 = done_bar + 8, qempty0 = qfull0 + 8 * kQ;
+  // claims: the 16-byte answer and its barrier, 512 bytes into the 1 KB after the staging rows
+  const uint32_t answer = smem_u32(bars) + 512, claim_bar = answer + 16;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 5 + 2 * kQ);
   int* s_item = reinterpret_cast<int*>(tmem_slot + 1);      // kQ x {item, start, end}
 
@@ -112,6 +114,7 @@ __global__ void __launch_bounds__(kTc64Threads, 1)
       mbar_init(tfull0 + 8 * b, 1);
       mbar_init(tempty0 + 8 * b, 4);
     }
+    mbar_init(claim_bar, 1);
     mbar_init(done_bar, 1);
     for (int q = 0; q < kQ; ++q) {
       mbar_init(qfull0 + 8 * q, 1);
@@ -153,9 +156,24 @@ __global__ void __launch_bounds__(kTc64Threads, 1)
       tma_prefetch_desc(&tmAg);
       tma_prefetch_desc(&tmA1);
       const uint64_t pol_a = l2_policy_evict_first();
+      // the next item: claimed as the current one starts, its answer read after
+      // the first group (dynamic), or a static stride
+      uint32_t claims = 0;
+      bool failed = false;
+      auto claim = [&] {
+        if (!p.dynamic) return;
+        fence_proxy_async_smem();   // the last answer has been read
+        mbar_arrive_expect_tx(claim_bar, 16);
+        clc_request(answer, claim_bar);
+      };
       auto next_item = [&](int cur) -> int {
-        int v = p.queue ? (int)atomicAdd(p.queue, 1u) : (cur < 0 ? (int)blockIdx.x : cur + (int)gridDim.x);
-        return v < p.n_items ? v : -1;
+        if (!p.dynamic) return cur + (int)gridDim.x < p.n_items ? cur + (int)gridDim.x : -1;
+        if (!mbar_wait(claim_bar, claims++ & 1, p.timeout_ns)) {
+          atomicOr(p.err, 4u);
+          failed = true;
+          return -1;
+        }
+        return clc_block(answer);
       };
       // block range of an item: its block row's range
       auto range = [&](int v, int* s0, int* s1) {
@@ -168,8 +186,7 @@ __global__ void __launch_bounds__(kTc64Threads, 1)
         *s1 = __ldg(p.row_ptr + row + 1);
       };
       uint32_t gs = 0, it = 0;
-      bool failed = false;
-      int item = next_item(-1);
+      int item = (int)blockIdx.x;   // the grid never exceeds the item count
       int start = 0, end = 0;
       range(item, &start, &end);
       for (;; ++it) {
@@ -183,10 +200,13 @@ __global__ void __launch_bounds__(kTc64Threads, 1)
         s_item[3 * q + 2] = end;
         mbar_arrive(qfull0 + 8 * q);
         if (item < 0 || failed) break;
-        const int nitem = next_item(item);
-        int nstart = 0, nend = 0;
-        range(nitem, &nstart, &nend);
+        claim();
+        int nitem = -2, nstart = 0, nend = 0;
         for (int j0 = start; j0 < end; j0 += G, ++gs) {
+          if (j0 > start && nitem == -2) {
+            nitem = next_item(item);
+            range(nitem, &nstart, &nend);
+          }
           const int n = min(G, end - j0);
           const int s = (int)(gs % STAGES);
           if (gs >= (uint32_t)STAGES && !mbar_wait(empty0 + 8 * s, ((gs / STAGES) + 1) & 1, p.timeout_ns)) {
@@ -210,18 +230,14 @@ __global__ void __launch_bounds__(kTc64Threads, 1)
             }
           }
         }
+        if (nitem == -2) {   // (after a failure too: an answer may still be on its way)
+          nitem = next_item(item);
+          range(nitem, &nstart, &nend);
+        }
         if (failed) break;
         item = nitem;
         start = nstart;
         end = nend;
-      }
-      if (p.queue) {
-        __threadfence();
-        if (atomicAdd(p.queue + 1, 1u) == gridDim.x - 1) {
-          p.queue[0] = 0;
-          p.queue[1] = 0;
-          __threadfence();
-        }
       }
     }
     __syncwarp();
@@ -514,15 +530,15 @@ spmm_status launch_tc64(const LaunchRequest& r) {
   p.timeout_ns = wait_limit_ns();
   p.err = r.err_word ? r.err_word : device_error_word();
   p.panel3d = panel3d;
-  p.queue = r.queue ? r.queue : (r.cfg.schedule == 1 ? work_queue_slot() : nullptr);
+  p.dynamic = r.cfg.schedule == 1 ? 1 : 0;
   if (!p.err) return fail(SPMM_ERR_CUDA, "could not set up the device error word");
   if (p.n_items == 0) return SPMM_OK;
   SPMM_CUDA_TRY(ensure_smem_attr(reinterpret_cast<const void*>(e->fn), (int)e->smem));
   long long grid = sm_count();
-  if (grid > p.n_items) grid = p.n_items;
+  if (grid > p.n_items || p.dynamic) grid = p.n_items;
   if (std::getenv("SPMM_DEBUG"))
-    std::fprintf(stderr, "[spmm] tcgen05-64 nt=%d stages=%d acc=%d group=%d smem=%zu grid=%lld items=%d queue=%d\n",
-                 nt, e->stages, e->acc, e->group, e->smem, grid, p.n_items, p.queue != nullptr);
+    std::fprintf(stderr, "[spmm] tcgen05-64 nt=%d stages=%d acc=%d group=%d smem=%zu grid=%lld items=%d dynamic=%d\n",
+                 nt, e->stages, e->acc, e->group, e->smem, grid, p.n_items, p.dynamic);
   SPMM_CUDA_TRY(launch_kernel(e->fn, dim3((unsigned)grid), dim3(kTc64Threads), e->smem, r.stream, tmA1, tmAg, tmAlo1,
                               tmAlog, tmB, tmBlo, p));
   return SPMM_OK;

@@ -42,11 +42,6 @@ __device__ __forceinline__ void umma_mxf8_scaled(uint32_t d_tmem, uint64_t a_des
 __device__ __forceinline__ void tmem_cp_32x128b_x4(uint32_t taddr, uint64_t s_desc) {
   asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(s_desc) : "memory");
 }
-// Generic-proxy shared-memory writes made visible to the async proxy (TMA,
-// tcgen05.mma / tcgen05.cp operand reads).
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");

@@ -4,10 +4,10 @@
 // The table has 56 entries:
 //   * five mma.sync tiles (column tile x ring depth);
 //   * 32 variants of the 128-column tcgen05 pipeline (column tile, ring depth,
-//     TMEM accumulators, static or work-queue schedule, split-K of 1, 2, 4
+//     TMEM accumulators, static or dynamic schedule, split-K of 1, 2, 4
 //     and, for the default 256-column tile, 8);
 //   * eight with a four-group ring and one accumulator (256 and 512 columns,
-//     static or queue, split-K 1 or 2), which only e4m3 instantiates (four
+//     static or dynamic, split-K 1 or 2), which only e4m3 instantiates (four
 //     blocks per group share one scale tile);
 //   * four of the 64-row pipeline (column tile x schedule);
 //   * seven per-matrix plans (schedule 2) on the tcgen05 shapes without
@@ -95,23 +95,9 @@ spmm_status spmm_config_supported(int bR, spmm_dtype dtype, int N, const spmm_co
 
 spmm_status spmm_default_config(int bR, spmm_dtype dtype, int N, spmm_config* out) {
   if (!out) return fail(SPMM_ERR_INVALID_ARG, "null config");
-  spmm_config c;
-  std::memset(&c, 0, sizeof(c));
-  // spmm_bcsr_mm with no configuration: the tcgen05 pipeline for 64-row
-  // blocks where it has a kernel (its first instantiation for the column tile:
-  // two accumulators, static schedule), else the mma.sync pipeline (depth 4).
-  // E4M3 stays on mma.sync, which takes any fp32 block scale (the tcgen05
-  // e4m3 kernels need powers of two).
-  if (bR == 64 && dtype != SPMM_E4M3 && tc_supported(bR, dtype, N, c)) {
-    c.kernel = 2;
-    c.n_tile = N <= 128 ? 128 : 256;
-    c.acc_buffers = 2;
-    c.split_k = 1;
-  } else {
-    c.kernel = 1;
-    c.n_tile = mma_default_nt(bR, dtype, N);
-    c.stages = 4;
-  }
+  // spmm_bcsr_mm with no configuration, the number of rows and of stored blocks
+  // not known
+  const spmm_config c = default_config(bR, dtype, 0, N, -1);
   *out = c;
   return spmm_config_supported(bR, dtype, N, &c) == SPMM_OK ? SPMM_OK
                                                             : fail(SPMM_ERR_UNSUPPORTED, "no default kernel");
