@@ -76,17 +76,28 @@ static_assert(sizeof(RingRec) == 64, "ring record");
 constexpr int kBatchThreads = 352;   // 11 warps, the roles of the single-product pipeline
 constexpr int kMaxBR = 64, kMaxNT = 256;
 
+// G = 0: groups of four 16- or 32-row blocks or of three 64-row ones, so that a
+// slot (36 KB) is about filled whatever the item's block height, and three
+// slots hold 12 blocks in flight, 9 of 64 rows. Fixed groups size a slot for
+// 64-row blocks and hold 8 of any height: 7040^2 in 16-row blocks, 25 %, N 512
+// took 64 us (two groups of four; 71 with four of two) and takes 54, the 64
+// products of the uneven workload 208 and take 185.
 template <int STAGES, int G>
 struct BatchCfg {
   static constexpr int kBoxBytes = 16 * 128;
   static constexpr int kPanelBytes = (kMaxNT / 64) * kBoxBytes;   // slot stride of one panel
+  // a slot: the group's A blocks (kAStage bytes, or for G = 0 what they take), then its panels
   static constexpr int kAStage = ((G * kMaxBR * 32 + 1023) / 1024) * 1024;
-  static constexpr int kStage = kAStage + G * kPanelBytes;
+  static constexpr int kStage = G > 0 ? kAStage + G * kPanelBytes : 4 * (32 * 32 + kPanelBytes);
   static constexpr int kAccCols = (kMaxNT / 128) * kMaxBR;          // 128
   static constexpr int kTmemCols = 2 * kAccCols;                     // two accumulators
   static constexpr int kQ = 4;
   static constexpr size_t kSmem = 1024 + (size_t)STAGES * kStage + 1024;
-  static_assert(G * kMaxBR <= 256 && 32 % G == 0, "a group is one TMA box and never straddles an index chunk");
+  static_assert(G == 0 || (G * kMaxBR <= 256 && 32 % G == 0), "a group is one TMA box and never straddles an index chunk");
+  static_assert(kStage % 1024 == 0, "swizzle atoms");
+  __host__ __device__ static constexpr int group(int bR) { return G > 0 ? G : bR == 64 ? 3 : 4; }
+  __device__ static constexpr int a_bytes(int bR) { return G > 0 ? kAStage : group(bR) * bR * 32; }   // 2, 4 or 6 KB
+  __device__ static constexpr int chunk(int bR) { return G == 0 && bR == 64 ? 30 : 32; }   // indices staged at a time: whole groups
 };
 
 template <int STAGES, int G, bool BF16>
@@ -209,8 +220,9 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_bcsr_tc_batch(const BatchP
         const BatchProblemDev* pr = p.probs + cur.prob;
         const int bR = cur.bR;
         const uint32_t blk_bytes = (uint32_t)(bR * 32 + cur.ntp * 32);
-        for (int j0 = cur.start; j0 < cur.end; j0 += G, ++gs) {
-          const int n = min(G, cur.end - j0);
+        const int g = Cfg::group(bR);
+        for (int j0 = cur.start; j0 < cur.end; j0 += g, ++gs) {
+          const int n = min(g, cur.end - j0);
           const int s = (int)(gs % STAGES);
           if (gs >= (uint32_t)STAGES && !mbar_wait(empty0 + 8 * s, ((gs / STAGES) + 1) & 1, p.timeout_ns)) {
             atomicOr(p.err, 4u);
@@ -223,7 +235,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_bcsr_tc_batch(const BatchP
           const int y0 = j0 * bR;
           if (cur.stk > 1) {
             // a stacked problem's member blocks are copied by the B issuers
-          } else if (n == G) {
+          } else if (n == g) {
             tma_tile_2d_g2s(smem_u32(a_dst), &pr->tmAg, 0, y0, fb, pol_a);
           } else {
             for (int b = 0; b < n; ++b)
@@ -264,6 +276,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_bcsr_tc_batch(const BatchP
       auto issue_blocks = [&](auto stacked_tag) {
         constexpr bool kStacked = decltype(stacked_tag)::value;
         const int stk = rec.stk;
+        const int g = Cfg::group(rec.bR), chunk = Cfg::chunk(rec.bR);
         const int* smap = kStacked ? pr->smap : nullptr;
         const int mbR = kStacked ? __ldg(&pr->mbR) : 0, oob = kStacked ? __ldg(&pr->oob_row) : 0;
         auto load_members = [&](int j, int (&mm)[4]) {
@@ -273,15 +286,16 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_bcsr_tc_batch(const BatchP
         int mym[4] = {-1, -1, -1, -1};
         if constexpr (kStacked) load_members(rec.start + lane, mym);
         int mycol = lane < rec.end - rec.start ? __ldg(rec.col_idx + rec.start + lane) : 0;
-        for (int base = rec.start; base < rec.end && !failed; base += 32) {
-          const int cnt = min(32, rec.end - base);
+        for (int base = rec.start; base < rec.end && !failed; base += chunk) {
+          const int cnt = min(chunk, rec.end - base);
           const int cur = mycol;
           int curm[4] = {mym[0], mym[1], mym[2], mym[3]};
           if constexpr (kStacked)
-            if (base + 32 < rec.end) load_members(base + 32 + lane, mym);
-          if (base + 32 < rec.end) mycol = lane < rec.end - base - 32 ? __ldg(rec.col_idx + base + 32 + lane) : 0;
-          for (int i0 = 0; i0 < cnt; i0 += G, ++gs) {
-            const int n = min(G, cnt - i0);
+            if (base + chunk < rec.end) load_members(base + chunk + lane, mym);
+          if (base + chunk < rec.end)
+            mycol = lane < rec.end - base - chunk ? __ldg(rec.col_idx + base + chunk + lane) : 0;
+          for (int i0 = 0; i0 < cnt; i0 += g, ++gs) {
+            const int n = min(g, cnt - i0);
             const int s = (int)(gs % STAGES);
             // Wait for the slot only in groups this issuer copies into: such a
             // group cannot be released without its bytes, so the slot's empty
@@ -296,7 +310,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_bcsr_tc_batch(const BatchP
             }
             failed = __shfl_sync(0xffffffffu, bad, 0);
             if (failed) break;
-            uint8_t* b_dst0 = smem + (size_t)s * Cfg::kStage + Cfg::kAStage;
+            uint8_t* b_dst0 = smem + (size_t)s * Cfg::kStage + Cfg::a_bytes(rec.bR);
             for (int b = bidx; b < n; b += kBIssuers) {
               const int col = __shfl_sync(0xffffffffu, cur, i0 + b);
               int src[4] = {-1, -1, -1, -1};
@@ -361,8 +375,9 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_bcsr_tc_batch(const BatchP
         }
         tc_fence_after();
         const uint32_t d0 = tmem + acc * Cfg::kAccCols;
-        for (int j0 = rec.start; j0 < rec.end; j0 += G, ++gs) {
-          const int n = min(G, rec.end - j0);
+        const int g = Cfg::group(bR);
+        for (int j0 = rec.start; j0 < rec.end; j0 += g, ++gs) {
+          const int n = min(g, rec.end - j0);
           const int s = (int)(gs % STAGES);
           if (!mbar_wait(full0 + 8 * s, (gs / STAGES) & 1, p.timeout_ns)) {
             atomicOr(p.err, 8u);
@@ -371,7 +386,7 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_bcsr_tc_batch(const BatchP
           }
           tc_fence_after();
           const uint32_t a_slot = smem_u32(smem + (size_t)s * Cfg::kStage);
-          const uint32_t b_slot = a_slot + Cfg::kAStage;
+          const uint32_t b_slot = a_slot + Cfg::a_bytes(bR);
           for (int b = 0; b < n; ++b) {
             const uint32_t b_addr = b_slot + b * Cfg::kPanelBytes;
             const uint64_t blk = smem_desc(a_slot + b * bR * 32, 16, 256, kLayoutSW32);
@@ -452,15 +467,15 @@ struct BatchEntry {
 };
 #define SPMM_BATCH_ENTRY(ST, G, BF) \
   BatchEntry{ST, G, BF, &k_bcsr_tc_batch<ST, G, BF>, BatchCfg<ST, G>::kSmem}
-// (ring depth in groups, blocks per group); the first entry per type is the default,
-// and the 4-stage one the default of a batch with stacked problems. All three hold
-// eight blocks in flight; two groups of four take half the barrier round trips of
-// four groups of two and ran the 64-product uneven batch faster with stacking off
-// (188 against 192 us); with stacking on, four groups of two ran it in 151 against
-// 157 us (and a second seed's 64 products in 257 against 274 us).
+// (ring depth in groups, blocks per group, 0: by block height); the first entry
+// per type is the default, the others are there on request. (The order of the
+// items was tried too: interleaving those bound by shared memory with those
+// that mostly write C, at the rate that spends both budgets evenly, 188 us
+// against 185 heaviest first.)
 const BatchEntry kBatchEntries[] = {
-    SPMM_BATCH_ENTRY(2, 4, false), SPMM_BATCH_ENTRY(4, 2, false), SPMM_BATCH_ENTRY(8, 1, false),
-    SPMM_BATCH_ENTRY(2, 4, true),  SPMM_BATCH_ENTRY(4, 2, true),  SPMM_BATCH_ENTRY(8, 1, true),
+    SPMM_BATCH_ENTRY(3, 0, false), SPMM_BATCH_ENTRY(2, 4, false), SPMM_BATCH_ENTRY(4, 2, false),
+    SPMM_BATCH_ENTRY(8, 1, false), SPMM_BATCH_ENTRY(3, 0, true),  SPMM_BATCH_ENTRY(2, 4, true),
+    SPMM_BATCH_ENTRY(4, 2, true),  SPMM_BATCH_ENTRY(8, 1, true),
 };
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -543,7 +558,7 @@ spmm_status spmm_batch_plan_create(const spmm_problem* problems, int count, cons
   const BatchEntry* e = nullptr;
   for (const BatchEntry& x : kBatchEntries) {
     if (x.bf16 != (dtype == SPMM_BF16)) continue;
-    if (c.stages > 0 && x.stages != c.stages) continue;
+    if (c.stages > 0 && (x.group == 0 || x.stages != c.stages)) continue;
     e = &x;
     break;
   }
@@ -696,16 +711,11 @@ spmm_status spmm_batch_plan_create(const spmm_problem* problems, int count, cons
     free_plan(plan);
     return fail(SPMM_ERR_UNSUPPORTED, "batched launch: too many items");
   }
-  // A batch with stacked problems defaults to four groups of two: each stacked
-  // block is up to four member copies, and the deeper ring keeps more of them
-  // in flight.
-  if (c.stages == 0 && plan->stacked > 0)
-    for (const BatchEntry& x : kBatchEntries)
-      if (x.bf16 == e->bf16 && x.stages == 4) e = &x;
   plan->entry = e;
   for (const GroupMap& g : group_maps) {
     spmm_status st = encode_tile_map_2d(&probs[g.prob].tmAg, CU_TENSOR_MAP_DATA_TYPE_UINT16, g.vals, 16, g.rows, 32,
-                                        16, (uint32_t)(e->group * g.bR), CU_TENSOR_MAP_SWIZZLE_32B);
+                                        16, (uint32_t)((e->group > 0 ? e->group : BatchCfg<3, 0>::group(g.bR)) * g.bR),
+                                        CU_TENSOR_MAP_SWIZZLE_32B);
     if (st != SPMM_OK) {
       free_plan(plan);
       return st;
