@@ -311,7 +311,7 @@ spmm_status spmm_hcsr_mm(const spmm_bcsr_desc* A_blocks, const spmm_csr_desc* A_
  * blocks (16 entries of one 16-row block row each, as a 16 x 16 block whose
  * column c holds entry c, plus the entries' 16 B-row indices). The tcgen05
  * pipeline then runs stored and gather blocks alike on the tensor cores, and
- * fetches a gather block's B rows with TMA tile::gather4. 16 x 16 fp16 blocks.
+ * fetches a gather block's B rows with cp.async. 16 x 16 fp16 blocks.
  * _create reads both parts on the device and synchronises `stream` once (for
  * the sizes). The plan owns its arrays: the parts may be freed after _create.
  * _run only launches (one kernel; no allocation or synchronisation); any N,

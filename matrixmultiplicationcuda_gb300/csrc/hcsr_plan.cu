@@ -7,9 +7,9 @@
 // block's B panel row c is B's row k (the entry's column). So
 //     block x panel = sum over the 16 entries of v * B[k][:] in row r,
 // exactly the CSR terms, in one UMMA per 128 output columns. The panel rows
-// are fetched with TMA tile::gather4 (four B rows per copy); unused slots of a
-// block row's last gather block have value 0 and row index K, which lies past
-// the end of B and reads zeros, so they add exact zeros.
+// are copied by the pipeline's B-issuing warps (cp.async, 16 bytes a lane);
+// unused slots of a block row's last gather block have value 0 and row index K,
+// which stands for a row of zeros, so they add exact zeros.
 //
 // The packed matrix is one BCSR matrix with 16 x 16 blocks: per block row, its
 // stored blocks (copied from the BCSR part) followed by its gather blocks,

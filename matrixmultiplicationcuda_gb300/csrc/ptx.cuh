@@ -28,6 +28,9 @@ __device__ __forceinline__ void fence_mbar_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
@@ -141,6 +144,15 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+// 16 bytes, or 16 zero bytes (src is not read then)
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool read) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(read ? 16 : 0) : "memory");
+}
+// Arrives on the mbarrier (one of its expected arrivals) once all this thread's
+// earlier cp.async copies have completed.
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ---- TMA -----------------------------------------------------------------------
@@ -160,18 +172,6 @@ __device__ __forceinline__ void tma_tile_2d_g2s(uint32_t dst, const void* tmap, 
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
       ".L2::cache_hint [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst),
       "l"(tmap), "r"(x), "r"(y), "r"(bar), "l"(policy)
-      : "memory");
-}
-// Four rows y0..y3 of a 2-D tensor, columns [x, x + box width), global -> shared
-// (tile::gather4; the map's box is one row high). The rows land one after the
-// other at dst with the map's swizzle, as rows of one taller box would. A row
-// outside the tensor reads the fill value (zeros).
-__device__ __forceinline__ void tma_gather4_g2s(uint32_t dst, const void* tmap, int x, int y0, int y1, int y2,
-                                                int y3, uint32_t bar, uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes"
-      ".L2::cache_hint [%0], [%1, {%2, %3, %4, %5, %6}], [%7], %8;" ::"r"(dst),
-      "l"(tmap), "r"(x), "r"(y0), "r"(y1), "r"(y2), "r"(y3), "r"(bar), "l"(policy)
       : "memory");
 }
 // Tiled 3-D tensor copy global -> shared; {x, y, z} innermost first.

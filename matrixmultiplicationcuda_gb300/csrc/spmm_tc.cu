@@ -74,6 +74,7 @@ struct TcParams {
   // planned hybrid product: a block with col_idx = -(g + 1) is a gather block,
   // whose panel rows are B rows gather_rows[16g .. 16g + 15] (NULL: none)
   const int* gather_rows;
+  int K;                  // rows of B: a gather index of K stands for a row of zeros
   // planned product (items NULL: item v is block row v / (ntiles * split)):
   // item v = items[v] = {block row, column tile, first block, end block}.
   // pair[v] = -1, or 128 * g + q for part q of split row (and tile) g, which
@@ -137,6 +138,7 @@ template <int BR, int NT, int STAGES, int MODE, int ACC, int G>
 struct TcCfg {
   static constexpr bool kSplit = MODE == MODE_SPLIT;
   static constexpr bool kE4 = MODE == MODE_E4M3;
+  static constexpr bool kGatherable = MODE == MODE_F16 && BR == 16;   // the planned hybrid product's matrices
   // a stacked plan's 64-row blocks are assembled from member blocks (fp16 / bf16)
   static constexpr bool kStackable = (MODE == MODE_F16 || MODE == MODE_BF16) && BR == 64;
   static constexpr int kParts = kSplit ? 2 : 1;
@@ -220,11 +222,13 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   const uint32_t answer = smem_u32(bars) + 512, claim_bar = answer + 16;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool gather = Cfg::kGatherable && p.gather_rows != nullptr;
   if (threadIdx.x == 32) {
     for (int s = 0; s < STAGES; ++s) {
       // the lead's arrive (it expects the whole group's bytes); e4m3 also B
       // issuer 0's, after it has written the group's scale tiles
-      mbar_init(full0 + 8 * s, Cfg::kE4 ? 2 : 1);
+      // (with gather blocks: every lane of every B issuer, in every group)
+      mbar_init(full0 + 8 * s, Cfg::kE4 ? 2 : gather ? 1 + 32 * kBIssuers : 1);
       mbar_init(empty0 + 8 * s, Cfg::kIssuers);   // each MMA issuer's commit
     }
     for (int b = 0; b < 2; ++b) {
@@ -453,7 +457,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             break;
           }
           const uint32_t fb = full0 + 8 * s;
-          mbar_arrive_expect_tx(fb, (uint32_t)(n * (Cfg::kABytes + Cfg::kPanelBytes) * Cfg::kParts));
+          // (with gather blocks the B issuers expect their panels' bytes themselves)
+          mbar_arrive_expect_tx(fb, (uint32_t)(n * (Cfg::kABytes + (gather ? 0 : Cfg::kPanelBytes)) * Cfg::kParts));
           uint8_t* a_dst = smem + (size_t)s * Cfg::kStage;
           const int y0 = j0 * BR;
           if constexpr (Cfg::kE4) {
@@ -525,8 +530,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       // stacked block, its member blocks from A's values into the block's A
       // slot; the two cases are separate instantiations, so the plain path
       // carries none of the member work.
-      auto issue_item = [&](auto stacked_tag) {
+      auto issue_item = [&](auto stacked_tag, auto gather_tag) {
         constexpr bool kStacked = decltype(stacked_tag)::value;
+        constexpr bool kGather = decltype(gather_tag)::value;
         // member blocks take the lead's policy for A
         const uint64_t pol_a = kStacked ? l2_policy_evict_first() : 0ull;
         int mycol = lane < end - start ? __ldg(p.col_idx + start + lane) : 0;
@@ -544,6 +550,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         if constexpr (Cfg::kE4) {
           if (bidx == kScaleWriter) mysc = lane < end - start ? __ldg(p.scales + start + lane) : 1.f;
         }
+        // gather blocks: lane r < 16 has B row r of gather block next_g (< 0: none)
+        [[maybe_unused]] int next_g = -1, next_rows = 0;
         for (int base = start; base < end && !failed; base += 32) {
           const int cnt = min(32, end - base);
           const int cur = mycol;
@@ -572,8 +580,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             // last, partial group, and the lead publishes an item once the group
             // 2 * STAGES before its first has been consumed (claim_ahead = STAGES - 1).
             // (Rotating the block-to-issuer map over groups of fewer than four
-            // blocks breaks this and was measured to corrupt a slot.)
-            const bool writes = bidx < n || (Cfg::kE4 && bidx == kScaleWriter);
+            // blocks breaks this and was measured to corrupt a slot.) With gather
+            // blocks every issuer arrives in every group, so every one waits.
+            const bool writes = kGather || bidx < n || (Cfg::kE4 && bidx == kScaleWriter);
             int bad = 0;
             if (lane == 0 && writes && gs >= (uint32_t)STAGES &&
                 !mbar_wait(empty0 + 8 * s, ((gs / STAGES) + 1) & 1, p.timeout_ns)) {
@@ -582,6 +591,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             }
             failed = __shfl_sync(0xffffffffu, bad, 0);
             if (failed) break;
+            if constexpr (kGather) __syncwarp();   // every lane writes into the slot that lane 0 saw free
             uint8_t* b_dst0 = smem + (size_t)s * Cfg::kStage + Cfg::kAStage;
             for (int b = bidx; b < n; b += kBIssuers) {
               const int col = __shfl_sync(0xffffffffu, cur, i0 + b);
@@ -590,27 +600,56 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 #pragma unroll
                 for (int t = 0; t < 4; ++t) src[t] = __shfl_sync(0xffffffffu, curm[t], i0 + b);
               }
-              if constexpr (!Cfg::kSplit && !Cfg::kE4 && !kStacked) {
-                if (col < 0 && p.gather_rows) {
-                  // Gather block: its panel is 16 arbitrary B rows. Lane L < 4 * (NT / 64)
-                  // copies rows 4q .. 4q + 3 (q = L % 4) of 64-column box L / 4 with one
-                  // tile::gather4 (tmBlo is then the one-row-box view of B), into the
-                  // box's rows 4q .. 4q + 3: the image of a 16-row box copy. Padding
-                  // rows index K, past the end of B, and read zeros.
-                  const long long g = -(long long)col - 1;
-                  const int kk = lane < 16 ? __ldg(p.gather_rows + 16 * g + lane) : 0;
-                  const int q = lane & 3;
-                  const int y0 = __shfl_sync(0xffffffffu, kk, 4 * q);
-                  const int y1 = __shfl_sync(0xffffffffu, kk, 4 * q + 1);
-                  const int y2 = __shfl_sync(0xffffffffu, kk, 4 * q + 2);
-                  const int y3 = __shfl_sync(0xffffffffu, kk, 4 * q + 3);
-                  if (lane < 4 * (NT / 64)) {
-                    const int bx = lane >> 2;
-                    tma_gather4_g2s(smem_u32(b_dst0 + (size_t)b * Cfg::kPanelBytes + bx * Cfg::kBoxBytes + q * 512),
-                                    &tmBlo, nt * NT + bx * 64, y0, y1, y2, y3, full0 + 8 * s, pol_b);
+              if constexpr (kGather) {
+                // The indices of this issuer's next gather block load while it
+                // copies the present one (after a gather block a row has only
+                // gather blocks, numbered upwards).
+                const int g = -col - 1;
+                int rows = next_rows;
+                if (col < 0 && next_g != g) rows = lane < 16 ? __ldg(p.gather_rows + 16ll * g + lane) : 0;
+                next_g = -1;
+                if (col < 0 && base + i0 + b + G < end)
+                  next_g = g + G;
+                else if (i0 + b + G < cnt)
+                  next_g = -__shfl_sync(0xffffffffu, cur, i0 + b + G) - 1;
+                if (next_g >= 0) next_rows = lane < 16 ? __ldg(p.gather_rows + 16ll * next_g + lane) : 0;
+                if (col < 0) {
+                  // Gather block: its panel is 16 arbitrary B rows, copied 16 bytes a
+                  // lane (a row's 256 columns per instruction) to where a 16-row box
+                  // copy with its 128-byte swizzle puts them. Index K is a row of zeros;
+                  // only a block row's last block has one, so the others' copies carry
+                  // no condition (with it and an L2 policy on each, the product below
+                  // took 101 us). TMA's tile::gather4 takes 16 copies of one issuing
+                  // thread for the same panel. 4096^2, 10 % stored blocks and 2 %
+                  // scattered entries (6532 stored, 19056 gather blocks), N 1024: 101 us
+                  // with gather4, 73 us now. A panel of gathered rows costs 220 cycles of
+                  // an SM, one TMA copies 161; shared memory alone takes 128 of either
+                  // (8 KB written, then read by the MMAs).
+                  uint8_t* b_dst = b_dst0 + (size_t)b * Cfg::kPanelBytes;
+                  const bool whole = __all_sync(0xffffffffu, lane >= 16 || rows < p.K);
+#pragma unroll
+                  for (int c0 = 0; c0 < NT / 8; c0 += 32) {
+                    // this lane's 8 columns of each row (past N: any columns, their results go nowhere)
+                    const int c = c0 + lane, n0 = nt * NT + 8 * c;
+                    const __half* src = p.Bh + (n0 < p.N ? n0 : 0);
+                    const uint32_t dst = smem_u32(b_dst + (c >> 3) * Cfg::kBoxBytes), sw = (uint32_t)(c & 7) << 4;
+                    if (whole) {
+#pragma unroll
+                      for (int r = 0; r < 16; ++r) {
+                        const unsigned row = (unsigned)__shfl_sync(0xffffffffu, rows, r);
+                        cp_async16(dst + r * 128 + (sw ^ ((r & 7) << 4)), src + (unsigned long long)row * (unsigned)p.ldb);
+                      }
+                    } else {
+                      for (int r = 0; r < 16; ++r) {
+                        const int row = __shfl_sync(0xffffffffu, rows, r);
+                        cp_async16_or_zero(dst + r * 128 + (sw ^ ((r & 7) << 4)),
+                                           src + (row < p.K ? (long long)row * p.ldb : 0), row < p.K);
+                      }
+                    }
                   }
                   continue;
                 }
+                if (lane == 0) mbar_expect_tx(full0 + 8 * s, Cfg::kPanelBytes);
               }
               if (lane == 0) {
                 const uint32_t fb = full0 + 8 * s;
@@ -644,6 +683,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
                 }
               }
             }
+            if constexpr (kGather) cp_async_arrive(full0 + 8 * s);
             if constexpr (Cfg::kE4) {
               if (bidx == kScaleWriter) {
                 // After its own copies are in flight: the group's 512-byte scale
@@ -671,12 +711,19 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       };
       if constexpr (Cfg::kStackable) {
         if (p.stk > 1) {
-          issue_item(std::true_type{});
+          issue_item(std::true_type{}, std::false_type{});
           continue;
         }
       }
-      issue_item(std::false_type{});
+      if constexpr (Cfg::kGatherable) {
+        if (gather) {
+          issue_item(std::false_type{}, std::true_type{});
+          continue;
+        }
+      }
+      issue_item(std::false_type{}, std::false_type{});
     }
+    if constexpr (Cfg::kGatherable) cp_async_wait_all();
   } else if (warp == 1 || (Cfg::kIssuers == 2 && warp == 10)) {
     // ------------------------------ MMA issuers ----------------------------------
     // Issuer i takes 128-column slices [i * kJPer, (i + 1) * kJPer) of every
@@ -708,6 +755,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             failed = true;
             break;
           }
+          if (gather) fence_proxy_async_smem();   // gathered rows are written by threads, not by TMA
           tc_fence_after();
           const uint32_t a_slot = smem_u32(smem + (size_t)s * Cfg::kStage);
           const uint32_t b_slot = a_slot + Cfg::kAStage;
@@ -1049,13 +1097,8 @@ spmm_status launch_tc(const LaunchRequest& r) {
   tmAlo1 = tmA1;
   tmAlog = tmAg;
   tmBlo = tmB;
-  if (r.gather_rows) {
-    // gather blocks: tmBlo becomes B viewed with a one-row box, the form tile::gather4 copies
-    if (mode == MODE_SPLIT) return fail(SPMM_ERR_UNSUPPORTED, "gather blocks run in fp16 or bf16");
-    st = encode_tile_map_2d(&tmBlo, CU_TENSOR_MAP_DATA_TYPE_UINT16, B.data, (uint64_t)r.N, (uint64_t)A.K,
-                            (uint64_t)B.ldb * 2, 64, 1, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (st != SPMM_OK) return st;
-  }
+  if (r.gather_rows && (mode != MODE_F16 || A.bR != 16))
+    return fail(SPMM_ERR_UNSUPPORTED, "gather blocks are 16 x 16 fp16 blocks");
   if (mode == MODE_SPLIT) {
     const void* lo = A.vals_lo ? A.vals_lo : B.data_lo;
     st = encode_tile_map_2d(&tmAlo1, CU_TENSOR_MAP_DATA_TYPE_UINT16, lo, 16, rows_bound, 32, 16,
@@ -1093,6 +1136,7 @@ spmm_status launch_tc(const LaunchRequest& r) {
   p.Bh = static_cast<const __half*>(B.data);
   p.ldb = B.ldb;
   p.gather_rows = r.gather_rows;
+  p.K = A.K;
   p.items = r.items;
   p.pair = r.pair;
   p.parts = r.parts;
