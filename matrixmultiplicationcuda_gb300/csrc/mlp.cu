@@ -492,7 +492,7 @@ struct ReduceParams {
   float* loss;
 };
 
-// grad = 2 / sum(mask) * (the CTAs' gradients, added in CTA order): blockIdx.y
+// grad = 2 / sum(mask) * (the CTAs' gradients, added in a fixed order): blockIdx.y
 // is the layer, a thread one weight or bias of it. mu and sigma are not
 // trained: their gradient is zero.
 __global__ void __launch_bounds__(128) k_mlp_reduce(const __grid_constant__ ReduceParams p) {
@@ -507,8 +507,17 @@ __global__ void __launch_bounds__(128) k_mlp_reduce(const __grid_constant__ Redu
   float s = 0.f;
   if (is_w || is_b) {
     const float* q = p.part + L.gpart + (is_w ? (k / I) * I4 + k % I : O4 * I4 + (k - O * I));
-#pragma unroll 16
-    for (int c = 0; c < p.ctas; ++c) s += q[(long long)c * stride];
+    for (int c0 = 0; c0 < p.ctas; c0 += 16) {
+      // 16 CTAs' sums in pairs: 12 roundings deep for 128 CTAs, not 128
+      float v[16];
+#pragma unroll
+      for (int c = 0; c < 16; ++c) v[c] = c0 + c < p.ctas ? q[(long long)(c0 + c) * stride] : 0.f;
+#pragma unroll
+      for (int d = 1; d < 16; d *= 2)
+#pragma unroll
+        for (int c = 0; c < 16; c += 2 * d) v[c] += v[c + d];
+      s += v[0];
+    }
   }
   if (threadIdx.x < 64) {
     // lanes add every 32nd CTA's sum, then a fixed tree: one order for all
