@@ -6,29 +6,24 @@ from typing import Optional
 
 import numpy as np
 
-from ._lib import (BcsrDesc, Config, DenseDesc, DType, SpmmError, Status, check, lib,
-                   stream_handle)
+from ._lib import (BcsrDesc, Config, CsrDesc, DenseDesc, DType, SpmmError, Status, check, lib,
+                   stream_handle, torch_module as _torch)
 
-_TORCH_DT = None
-
-
-def _torch():
-    import torch
-    return torch
-
-
-def _addr(t):
-    return None if t is None else t.data_ptr()
+# The calls below are short next to their kernels only if little Python runs in
+# each: descriptors are filled by position (a store per field costs 0.1 us) and
+# addresses go to the library as integers, which its signatures convert.
 
 
 def _ptr(t):
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def storage_dtype(dtype):
     torch = _torch()
-    return {DType.F16: torch.float16, DType.BF16: torch.bfloat16, DType.E4M3: torch.uint8,
-            DType.F16_SPLIT: torch.float16}[DType(dtype)]
+    dtype = DType(dtype)
+    if dtype is DType.BF16:
+        return torch.bfloat16
+    return torch.uint8 if dtype is DType.E4M3 else torch.float16
 
 
 @dataclass
@@ -55,15 +50,10 @@ class BCSR:
         return int(self.col_idx.numel())
 
     def desc(self):
-        d = BcsrDesc()
-        d.M, d.K, d.bR, d.bC = self.M, self.K, self.bR, self.bC
-        d.row_ptr = self.row_ptr.data_ptr()
-        d.col_idx = self.col_idx.data_ptr() if self.col_idx.numel() else None
-        d.vals = self.vals.data_ptr() if self.vals.numel() else None
-        d.vals_lo = self.vals_lo.data_ptr() if self.vals_lo is not None else None
-        d.scales = self.scales.data_ptr() if self.scales is not None else None
-        d.dtype = int(self.dtype)
-        return d
+        ci, v = self.col_idx, self.vals
+        return BcsrDesc(self.M, self.K, self.bR, self.bC, self.row_ptr.data_ptr(),
+                        ci.data_ptr() if ci.numel() else None, v.data_ptr() if v.numel() else None,
+                        _ptr(self.vals_lo), _ptr(self.scales), int(self.dtype))
 
     @staticmethod
     def from_host(M, K, bR, row_ptr, col_idx, vals_f32, dtype=DType.F16, device="cuda"):
@@ -78,12 +68,7 @@ class BCSR:
 
 
 def _dense_desc(B, B_lo=None, scale=1.0, ldb=None):
-    d = DenseDesc()
-    d.data = B.data_ptr()
-    d.data_lo = B_lo.data_ptr() if B_lo is not None else None
-    d.scale = float(scale)
-    d.ldb = int(ldb if ldb is not None else B.shape[-1])
-    return d
+    return DenseDesc(B.data_ptr(), _ptr(B_lo), float(scale), int(ldb if ldb is not None else B.shape[-1]))
 
 
 def spmm(A: BCSR, B, N=None, C=None, cfg: Optional[Config] = None, stream=None, B_lo=None,
@@ -96,7 +81,7 @@ def spmm(A: BCSR, B, N=None, C=None, cfg: Optional[Config] = None, stream=None, 
     ldc = int(C.stride(0)) if ldc is None else int(ldc)
     a = A.desc()
     b = _dense_desc(B, B_lo, b_scale, ldb=B.stride(0))
-    check(lib().spmm_bcsr_mm_nnzb(ctypes.byref(a), A.nnzb, ctypes.byref(b), N, ctypes.c_void_p(C.data_ptr()), ldc,
+    check(lib().spmm_bcsr_mm_nnzb(ctypes.byref(a), A.nnzb, ctypes.byref(b), N, C.data_ptr(), ldc,
                                   ctypes.byref(cfg) if cfg is not None else None, stream_handle(stream)))
     return C
 
@@ -106,7 +91,6 @@ def hcsr_mm(A_blocks: BCSR, csr_row_ptr, csr_col_idx, csr_vals, B, N=None, C=Non
     """Hybrid product C = A_blocks @ B + A_rest @ B in one launch (fp16): the
     BCSR part on the tensor cores, the CSR part (row_ptr [M+1], col_idx, fp16
     vals, device tensors) added in the same kernel's epilogue."""
-    from ._lib import CsrDesc
     torch = _torch()
     N = int(B.shape[1]) if N is None else int(N)
     if C is None:
@@ -119,7 +103,7 @@ def hcsr_mm(A_blocks: BCSR, csr_row_ptr, csr_col_idx, csr_vals, B, N=None, C=Non
     r.col_idx = csr_col_idx.data_ptr() if csr_col_idx.numel() else None
     r.vals = csr_vals.data_ptr() if csr_vals.numel() else None
     b = _dense_desc(B, None, 1.0, ldb=B.stride(0))
-    check(lib().spmm_hcsr_mm(ctypes.byref(a), ctypes.byref(r), ctypes.byref(b), N, ctypes.c_void_p(C.data_ptr()),
+    check(lib().spmm_hcsr_mm(ctypes.byref(a), ctypes.byref(r), ctypes.byref(b), N, C.data_ptr(),
                              ldc, ctypes.byref(cfg) if cfg is not None else None, stream_handle(stream)))
     return C
 
@@ -169,7 +153,7 @@ class BcsrPlan:
         a = A.desc()
         b = _dense_desc(B, B_lo, b_scale, ldb=B.stride(0))
         check(lib().spmm_bcsr_plan_run_ex(self._h, ctypes.byref(a), ctypes.byref(b), self.N,
-                                          ctypes.c_void_p(C.data_ptr()), ldc, RUN_INPUTS_READY if inputs_ready else 0,
+                                          C.data_ptr(), ldc, RUN_INPUTS_READY if inputs_ready else 0,
                                           stream_handle(stream)))
         return C
 
@@ -191,7 +175,6 @@ class HcsrPlan:
     The plan copies both parts; run() is one launch."""
 
     def __init__(self, A_blocks: BCSR, csr_row_ptr, csr_col_idx, csr_vals, stream=None):
-        from ._lib import CsrDesc
         a = A_blocks.desc()
         r = CsrDesc()
         r.M, r.K = A_blocks.M, A_blocks.K
@@ -216,7 +199,7 @@ class HcsrPlan:
             C = torch.empty((self.M, N), dtype=torch.float32, device=B.device)
         ldc = int(C.stride(0)) if ldc is None else int(ldc)
         b = _dense_desc(B, None, 1.0, ldb=B.stride(0))
-        check(lib().spmm_hcsr_plan_run(self._h, ctypes.byref(b), N, ctypes.c_void_p(C.data_ptr()), ldc,
+        check(lib().spmm_hcsr_plan_run(self._h, ctypes.byref(b), N, C.data_ptr(), ldc,
                                        ctypes.byref(cfg) if cfg is not None else None, stream_handle(stream)))
         return C
 
@@ -246,13 +229,12 @@ def dense_mm(A, B, C=None, stream=None):
         C = torch.empty((M, N), dtype=torch.float32, device=B.device)
     b = _dense_desc(B, None, 1.0, ldb=B.stride(0))
     check(lib().spmm_dense_mm(ctypes.c_void_p(A.data_ptr()), int(A.stride(0)), ctypes.byref(b), M, K, N, int(dt),
-                              ctypes.c_void_p(C.data_ptr()), int(C.stride(0)), stream_handle(stream)))
+                              C.data_ptr(), int(C.stride(0)), stream_handle(stream)))
     return C
 
 
 def csr_mm(row_ptr, col_idx, vals, K, B, N=None, C=None, stream=None, ldc=None):
     """CSR x dense (fp16, device tensors), C fp32: the native comparator."""
-    from ._lib import CsrDesc
     torch = _torch()
     N = int(B.shape[1]) if N is None else int(N)
     M = row_ptr.numel() - 1
@@ -264,7 +246,7 @@ def csr_mm(row_ptr, col_idx, vals, K, B, N=None, C=None, stream=None, ldc=None):
     r.col_idx = col_idx.data_ptr() if col_idx.numel() else None
     r.vals = vals.data_ptr() if vals.numel() else None
     b = _dense_desc(B, None, 1.0, ldb=B.stride(0))
-    check(lib().spmm_csr_mm(ctypes.byref(r), ctypes.byref(b), N, ctypes.c_void_p(C.data_ptr()),
+    check(lib().spmm_csr_mm(ctypes.byref(r), ctypes.byref(b), N, C.data_ptr(),
                             int(C.stride(0)) if ldc is None else int(ldc), stream_handle(stream)))
     return C
 
@@ -272,13 +254,11 @@ def csr_mm(row_ptr, col_idx, vals, K, B, N=None, C=None, stream=None, ldc=None):
 def _ref_launch(bR, hdr, idx, data, B, C, M, N, K, stream):
     """The reference-shaped call: contiguous fp16 operands given by their arrays
     (what the library's <name>_launch entries do, with the stored blocks known)."""
-    a = BcsrDesc()
-    a.M, a.K, a.bR, a.bC = int(M), int(K), bR, 16
-    a.row_ptr, a.col_idx, a.vals = _addr(hdr), _addr(idx), _addr(data)
-    b = DenseDesc()
-    b.data, b.scale, b.ldb = _addr(B), 1.0, int(N)
-    check(lib().spmm_bcsr_mm_nnzb(ctypes.byref(a), -1 if idx is None else idx.numel(), ctypes.byref(b), int(N),
-                                  _ptr(C), int(N), None, stream_handle(stream)))
+    N = int(N)
+    a = BcsrDesc(int(M), int(K), bR, 16, _ptr(hdr), _ptr(idx), _ptr(data))
+    b = DenseDesc(_ptr(B), None, 1.0, N)
+    check(lib().spmm_bcsr_mm_nnzb(a, -1 if idx is None else idx.numel(), b, N, _ptr(C), N, None,
+                                  stream_handle(stream)))
     return C
 
 

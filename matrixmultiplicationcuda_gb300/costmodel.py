@@ -47,7 +47,7 @@ def init_params(s, mu, sigma, seed=0):
 
 
 def _vp(t):
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 class MLP:
