@@ -375,14 +375,17 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       // under the inputs-ready promise a claim waits for the previous kernel,
       // and the copies of A's last groups would wait with it.
       const bool no_more = p.queue && (int)gridDim.x >= p.n_items;
-      // two instances, so that neither way of claiming costs the other instructions:
-      // a plan of short rows (7184 x 656, 16-row blocks, N 2432) took 20.7 us with one, 20.1 now
-      auto copy_items = [&](auto dynamic_tag) {
-        constexpr bool kDynamic = decltype(dynamic_tag)::value;
-        const bool late = (kDynamic || p.queue != nullptr) && p.claim_ahead >= 0 && !no_more;
+      // 16- and 32-row kernels: an instance per way of claiming, so that neither
+      // runs the other's tests (plans of 16 rows, 7184 x 656, N 2432: 20.7 us with
+      // one instance, 20.1 with two). In the 64-row kernels two cost more than the
+      // tests (a stacked plan, 8192^2 band, 16 rows, N 1024: 23.1 us and 23.6).
+      auto copy_items = [&](auto way) {
+        constexpr int kWay = decltype(way)::value;   // 1 = pending blocks, 0 = queue or stride, -1 = as p.dynamic says
+        const bool dynamic = kWay >= 0 ? kWay != 0 : p.dynamic != 0;
+        const bool late = (dynamic || p.queue != nullptr) && p.claim_ahead >= 0 && !no_more;
         uint32_t claims = 0;
         auto claim = [&]() -> unsigned {
-          if constexpr (!kDynamic) {
+          if (!dynamic) {
             if (!dep_waited) {
               grid_dep_wait();
               dep_waited = true;
@@ -395,7 +398,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
           return 0u;
         };
         auto claimed_item = [&](unsigned t) -> int {
-          if constexpr (!kDynamic) {
+          if (!dynamic) {
             const unsigned v = t + gridDim.x;
             return v < (unsigned)p.n_items ? (int)v : -1;
           }
@@ -425,7 +428,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
           if (!late) {
             // the next item's indices load now and are used once this item is copied
             nitem = no_more ? -1
-                    : kDynamic || p.queue ? claimed_item(claim())
+                    : dynamic || p.queue ? claimed_item(claim())
                                            : (item + (int)gridDim.x < p.n_items ? item + (int)gridDim.x : -1);
             range(nitem, &nstart, &nend, &ntile);
           }
@@ -483,7 +486,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             }
           }
           if (failed) {
-            if (kDynamic && claimed && nitem == -2) claimed_item(ticket);   // an answer still on its way
+            if (dynamic && claimed && nitem == -2) claimed_item(ticket);   // an answer still on its way
             break;
           }
           in_ring = late && nitem != -2;
@@ -498,10 +501,14 @@ __global__ void __launch_bounds__(kTcThreads, 2)
           tile = ntile;
         }
       };
-      if (p.dynamic)
-        copy_items(std::true_type{});
-      else
-        copy_items(std::false_type{});
+      if constexpr (BR == 64) {
+        copy_items(std::integral_constant<int, -1>{});
+      } else {
+        if (p.dynamic)
+          copy_items(std::integral_constant<int, 1>{});
+        else
+          copy_items(std::integral_constant<int, 0>{});
+      }
       // the last CTA to finish resets the queue for the next launch
       if (p.queue && !no_more) {
         if (!dep_waited) grid_dep_wait();
