@@ -92,8 +92,10 @@ const char* spmm_last_error(void);
  * written (rows whose block row is empty get zeros), so C need not be cleared.
  * N must be a multiple of 8 and ldb a multiple of 8 (16-byte TMA strides);
  * E4M3 needs multiples of 16. cfg may be NULL.
- * E4M3 with kernel 0 runs the mma.sync pipeline, which takes any fp32 block
- * scale. Kernel 2 runs the tcgen05 block-scaled kernels (kind::mxf8f6f4):
+ * E4M3 with kernel 0 runs the mma.sync pipeline or, for 32- and 64-row blocks
+ * and longer rows when the number of stored blocks is known (see below), the
+ * tcgen05 pipeline on e4m3 converted to fp16; both take any fp32 block scale.
+ * Kernel 2 runs the tcgen05 block-scaled kernels (kind::mxf8f6f4):
  * every block scale must be a positive normal power of two, as spmm_quantize
  * makes them (another scale raises a flag spmm_device_error_check reports);
  * each 16-wide block is a K = 32 MMA whose second half multiplies zeros by

@@ -300,7 +300,9 @@ namespace spmm {
 //     narrower products stay.
 //   split fp16, 64-row blocks above 128 columns: the 64-row pipeline (16384^2,
 //     2 %, N 512: 30.5 against 33.9 for tc256).
-//   e4m3: mma.sync, which takes any block scale.
+//   e4m3: mma.sync or, where converts_e4m3 says so, the tcgen05 pipeline with
+//     e4m3 converted to fp16; both take any block scale (the block-scaled MMA,
+//     which a caller may ask for, is faster but needs powers of two).
 spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnzb) {
   spmm_config c;
   std::memset(&c, 0, sizeof(c));
@@ -335,6 +337,24 @@ spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnz
   c.n_tile = bR == 64 && dtype != SPMM_E4M3 && dtype != SPMM_F16_SPLIT ? 64 : mma_default_nt(bR, dtype, N);
   c.stages = 4;
   return c;
+}
+
+// Whether an e4m3 product of known size runs converted to fp16 in the tcgen05
+// pipeline instead of on mma.sync (us, converted against mma.sync):
+//   64 rows: 16384^2, 2 % (20 blocks a row), N 512: 25.3, 34.3; 8192^2, 10 %, N
+//     1024: 47.6, 73.4; 32 rows: 60.9, 87.9; 8192^2 with log-normal rows, 3 %, N
+//     1024: 64 rows 32.4, 43.2, 32 rows 31.0, 44.4.
+//   Short rows do not fill its ring: 64 rows, 8192^2, 2 % (10 a row): 17.7, 19.9
+//     at N 1024, but 1 % (5 a row), N 512: 10.0, 9.2; 32 rows: 10.6, 9.5.
+//   With fewer items than CTAs run at once the longest rows bound both, and
+//     mma.sync's narrower tiles spread them further: 64 rows, 8192^2 with
+//     log-normal rows, N 512 (256 items): 45.6, 44.6.
+//   Its tile is 256 wide: 32 rows, 16384 x 8192, 5 %, N 272: 39.8, 35.8.
+//   16 rows: slower (8192^2, 10 %, N 1024: 108, 95 with mma.sync's 256-column tile).
+bool converts_e4m3(int bR, int M, int N, long long nnzb) {
+  if (bR == 16 || nnzb < 0 || N <= 128 || (N > 256 && N <= 384)) return false;
+  const long long items = (long long)(M / bR) * ((N + 255) / 256);
+  return nnzb * bR >= 10ll * M && items >= 2ll * sm_count();
 }
 
 }  // namespace spmm
@@ -393,12 +413,20 @@ spmm_status spmm_bcsr_mm_nnzb(const spmm_bcsr_desc* A, long long nnzb, const spm
                        want.schedule == 0 && want.split_k <= 1;
     if (plain) {
       r.cfg = default_config(A->bR, A->dtype, A->M, N, nnzb);
+      if (e4m3 && converts_e4m3(A->bR, A->M, N, nnzb)) {
+        r.convert = true;
+        r.cfg.kernel = 2;
+        r.cfg.n_tile = 256;
+        r.cfg.stages = 0;
+        r.cfg.schedule = 1;
+      }
     } else {
       r.cfg.kernel = A->bR == 64 && !e4m3 ? 2 : 1;
     }
     spmm_status st = r.cfg.kernel == 1 ? launch_mma(r) : r.cfg.kernel == 3 ? launch_tc64(r) : launch_tc(r);
     if (st != SPMM_ERR_UNSUPPORTED || r.cfg.kernel == 1) return st;
     g_last_error.clear();
+    r.convert = false;
     r.cfg = want;
     r.cfg.kernel = 0;
     return launch_mma(r);

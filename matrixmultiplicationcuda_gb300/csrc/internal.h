@@ -77,6 +77,9 @@ struct LaunchRequest {
   // stored and gather blocks
   const int* gather_rows = nullptr;
   long long total_blocks = 0;
+  // e4m3 converted to fp16 on the way into shared memory (any block scale),
+  // in place of the block-scaled MMA (powers of two)
+  bool convert = false;
   // planned product (kernel 2): the item list, split-row pairs and their
   // counters (see spmm_bcsr_plan_create)
   const int4* items = nullptr;

@@ -74,7 +74,7 @@ struct TcParams {
   // planned hybrid product: a block with col_idx = -(g + 1) is a gather block,
   // whose panel rows are B rows gather_rows[16g .. 16g + 15] (NULL: none)
   const int* gather_rows;
-  int K;                  // rows of B: a gather index of K stands for a row of zeros
+  int K;                  // rows of B (a gather index of K stands for a row of zeros)
   // planned product (items NULL: item v is block row v / (ntiles * split)):
   // item v = items[v] = {block row, column tile, first block, end block}.
   // pair[v] = -1, or 128 * g + q for part q of split row (and tile) g, which
@@ -107,6 +107,10 @@ __device__ __forceinline__ void st_release_gpu(unsigned* ptr, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(ptr), "r"(v) : "memory");
 }
 
+// Who writes a group's slot: TMA alone; the planned hybrid product's gather
+// blocks (B rows copied by the B issuers); e4m3 converted to fp16 by them.
+enum Feed : int { kFeedTma = 0, kFeedGather = 1, kFeedConvert = 2 };
+
 // BR: block height (the UMMA N); NT: output columns per item; STAGES: ring
 // depth in groups; ACC: TMEM accumulators per CTA (2 = one item's epilogue
 // overlaps the next item's MMAs inside the CTA; 1 = half the TMEM, so two CTAs
@@ -134,7 +138,7 @@ __device__ __forceinline__ void st_release_gpu(unsigned* ptr, unsigned v) {
 // which TMEM lanes the MMA reads. The panel side's factor is a constant 1
 // (0x7F), copied once per CTA and issuer. B's scale multiplies C
 // in the epilogue.
-template <int BR, int NT, int STAGES, int MODE, int ACC, int G>
+template <int BR, int NT, int STAGES, int MODE, int ACC, int G, int FEED = kFeedTma>
 struct TcCfg {
   static constexpr bool kSplit = MODE == MODE_SPLIT;
   static constexpr bool kE4 = MODE == MODE_E4M3;
@@ -166,7 +170,12 @@ struct TcCfg {
   static constexpr int kTailOff = kAStage + G * kPanelBytes * kParts;
   static constexpr int kStage = kE4 ? ((kTailOff + 2048 + 1023) / 1024) * 1024 : kTailOff;
   // e4m3, after the ring: the panel-side scale tile (512 bytes of 0x7F)
-  static constexpr int kExtra = kE4 ? 512 : 0;
+  // converted e4m3, after the ring: per B issuer, kDepth groups of raw bytes
+  // (16 of A and kCopies x 16 of B per lane, and the block's scale)
+  static constexpr int kDepth = STAGES;
+  static constexpr int kCopies = 16 * G / 4 * (NT / 16) / 32;
+  static constexpr int kRawGroup = (kCopies + 1) * 512 + 16;
+  static constexpr int kExtra = kE4 ? 512 : FEED == kFeedConvert ? 4 * kDepth * kRawGroup : 0;
   static constexpr int kAccCols = kJ * BR;            // TMEM columns of one accumulator
   // e4m3 scale factors in TMEM, per MMA issuer i: 4 columns for the panel
   // side (kSfaCol + 4 i), 4 per ring slot s (kSfbCol + 4 (i STAGES + s))
@@ -194,13 +203,16 @@ struct TcCfg {
 
 constexpr int kTcThreads = 352;   // 11 warps
 
-template <int BR, int NT, int STAGES, int MODE, int ACC, int G, bool GATHER = false>
+
+template <int BR, int NT, int STAGES, int MODE, int ACC, int G, int FEED = kFeedTma>
 __global__ void __launch_bounds__(kTcThreads, 2)
     k_bcsr_tc(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmAg,
               const __grid_constant__ CUtensorMap tmAlo1, const __grid_constant__ CUtensorMap tmAlog,
               const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmBlo,
               const TcParams p) {
-  using Cfg = TcCfg<BR, NT, STAGES, MODE, ACC, G>;
+  using Cfg = TcCfg<BR, NT, STAGES, MODE, ACC, G, FEED>;
+  constexpr int kASource = FEED == kFeedConvert ? BR * 16 : Cfg::kABytes;   // bytes of a block in A's values
+  constexpr bool GATHER = FEED == kFeedGather, CONVERT = FEED == kFeedConvert;
   constexpr int kQ = 4;                       // item hand-off ring depth
   constexpr int kBIssuers = 4;
   constexpr int kScaleWriter = 3;             // e4m3: the B issuer that writes the scale tiles
@@ -226,7 +238,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       // the lead's arrive (it expects the whole group's bytes); e4m3 also B
       // issuer 0's, after it has written the group's scale tiles
       // (with gather blocks: every lane of every B issuer, in every group)
-      mbar_init(full0 + 8 * s, Cfg::kE4 ? 2 : GATHER ? 1 + 32 * kBIssuers : 1);
+      // (converted e4m3: each B issuer, in every group)
+      mbar_init(full0 + 8 * s, Cfg::kE4 ? 2 : GATHER ? 1 + 32 * kBIssuers : CONVERT ? kBIssuers : 1);
       mbar_init(empty0 + 8 * s, Cfg::kIssuers);   // each MMA issuer's commit
     }
     for (int b = 0; b < 2; ++b) {
@@ -313,8 +326,10 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     // the ring slot, expects the group's bytes on its full barrier and copies the
     // A blocks. The B issuers copy the group's B panels into the same slot.
     if (lane == 0) {
-      tma_prefetch_desc(&tmAg);
-      tma_prefetch_desc(&tmA1);
+      if constexpr (!CONVERT) {
+        tma_prefetch_desc(&tmAg);
+        tma_prefetch_desc(&tmA1);
+      }
       const uint64_t pol_a = l2_policy_evict_first();
       uint32_t gs = 0, it = 0;
       bool failed = false;
@@ -439,7 +454,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             // 1-2 % on back-to-back plans of the headline product; no effect on
             // e4m3 or on a launch timed alone)
             if (end > start && p.stk <= 1)
-              tma_prefetch_l2(p.avals + (size_t)start * Cfg::kABytes, (uint32_t)((end - start) * Cfg::kABytes));
+              tma_prefetch_l2(p.avals + (size_t)start * kASource, (uint32_t)((end - start) * kASource));
           }
           int gi = 0;
           for (int j0 = start; j0 < end; j0 += G, ++gs, ++gi) {
@@ -461,6 +476,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
               failed = true;
               break;
             }
+            // (the B issuers convert A's blocks too; the wait above keeps the claims' pace)
+            if constexpr (CONVERT) continue;
             const uint32_t fb = full0 + 8 * s;
             // (with gather blocks the B issuers expect their panels' bytes themselves)
             mbar_arrive_expect_tx(fb, (uint32_t)(n * (Cfg::kABytes + (GATHER ? 0 : Cfg::kPanelBytes)) * Cfg::kParts));
@@ -527,10 +544,152 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     // the group's slot (a TMA copy holds its issuing thread for ~200 ns, so four
     // threads share the panels). Its lanes stage column indices 32 at a time,
     // prefetching the next chunk while lane 0 issues.
-    if (lane == 0) tma_prefetch_desc(&tmB);
+    if (!CONVERT && lane == 0) tma_prefetch_desc(&tmB);
     const uint64_t pol_b = l2_policy_evict_last();
     uint32_t gs = 0;
     int failed = 0;
+    // Converted e4m3: the issuers copy the raw bytes of their blocks and panels
+    // into staging of their own (cp.async, kDepth groups ahead, across items),
+    // convert them to fp16 (the block scale multiplied into A) and store them
+    // where TMA would have put fp16 ones. kPer issuers share a block of a
+    // group, each kRows of its panel's rows and kARows of its own. A lane reads
+    // back only what it copied, so the staging needs no barrier.
+    //
+    // The conversion bounds it: of the 1316 cycles that an issuer spends on a
+    // group of two 64-row blocks, 553 convert, 498 copy, 252 wait for the slot,
+    // while the MMA threads wait. Groups of four blocks (a whole panel per
+    // issuer) cost little more than groups of two: 32 rows, 8192^2, 10 %, N
+    // 1024: 61 us against 84; for 64 rows they do not fit twice on an SM. Eight
+    // converting warps: 27.8 us where four take 25.5 (16384^2, 64 rows, 2 %, N
+    // 512); TMA copies by one more warp, which then holds everyone up: 27.5.
+    [[maybe_unused]] auto convert_stream = [&]() {
+      constexpr int kDepth = Cfg::kDepth, kPer = kBIssuers / G, kRows = 16 / kPer, kARows = BR / kPer;
+      constexpr int kCopies = Cfg::kCopies;
+      static_assert(!CONVERT || (NT == 256 && kARows <= 32 && kBIssuers % G == 0), "the lane maps below");
+      const int myb = bidx / kPer, part = bidx % kPer;
+      // Lane: 16 columns (a 16-byte chunk c) of rows r0, r0 + 2, ...: eight lanes
+      // hold four chunks of two rows, whose fp16 stores fall on all banks.
+      const int c = (lane & 3) + 4 * (lane >> 3), r0 = part * kRows + ((lane >> 2) & 1);
+      const uint8_t* bsrc = reinterpret_cast<const uint8_t*>(p.Bh) + (long long)r0 * p.ldb;
+      const int arow = part * kARows + lane;
+      const uint8_t* asrc = p.avals + arow * 16;
+      const uint32_t a_off = arow * 32, a_sw = ((arow >> 2) & 1) << 4;
+      const uint32_t b_off = Cfg::kAStage + (c >> 2) * Cfg::kBoxBytes + r0 * 128;
+      const uint32_t raw0 = smem_u32(smem) + STAGES * Cfg::kStage + bidx * (kDepth * Cfg::kRawGroup);
+      // the copying end of the stream
+      uint32_t it = 0, copied = 0, has = 0;   // groups copied; bit g % 32: group g holds a block of this issuer
+      int j0 = 0, end = 0, base = 0, cols = 0, next_cols = 0;   // next group; lane's column indices from base, base + 32
+      const uint8_t* bcol = bsrc;
+      bool done = false;
+      auto copy_group = [&]() {
+        while (!done && j0 >= end) {
+          int item = -1, start = 0, e = 0, nt = 0, ok = 1;
+          if (lane == 0) ok = read_item(it, &item, &start, &e, 4u, &nt) ? 1 : 0;
+          ok = __shfl_sync(0xffffffffu, ok, 0);
+          item = __shfl_sync(0xffffffffu, item, 0);
+          j0 = base = __shfl_sync(0xffffffffu, start, 0);
+          end = __shfl_sync(0xffffffffu, e, 0);
+          nt = __shfl_sync(0xffffffffu, nt, 0);
+          ++it;
+          done = !ok || item < 0;
+          const int n0 = nt * NT + 16 * c;   // (past N: any columns, their results go nowhere)
+          bcol = bsrc + (n0 < p.N ? n0 : 0);
+          cols = base + lane < end && !done ? __ldg(p.col_idx + base + lane) : 0;
+          next_cols = base + 32 + lane < end && !done ? __ldg(p.col_idx + base + 32 + lane) : 0;
+        }
+        if (!done) {
+          if (j0 - base == 32) {
+            base = j0;
+            cols = next_cols;
+            next_cols = base + 32 + lane < end ? __ldg(p.col_idx + base + 32 + lane) : 0;
+          }
+          const int j = j0 + myb;
+          has &= ~(1u << (copied & 31));
+          if (j < end) {
+            has |= 1u << (copied & 31);
+            const int col = __shfl_sync(0xffffffffu, cols, j - base);
+            const uint32_t raw = raw0 + (copied % kDepth) * Cfg::kRawGroup + lane * 16;
+            if (lane < kARows) cp_async16(raw, asrc + (long long)j * (BR * 16));
+            if ((unsigned)col < (unsigned)(p.K >> 4)) {
+              const uint8_t* src = bcol + (long long)col * 16 * p.ldb;
+#pragma unroll
+              for (int k = 0; k < kCopies; ++k) cp_async16(raw + 512 * (k + 1), src + 2 * k * p.ldb);
+            } else {   // not a block column of A: rows of zeros, as a TMA copy reads them
+#pragma unroll
+              for (int k = 0; k < kCopies; ++k) st_shared_v4(raw + 512 * (k + 1), make_uint4(0u, 0u, 0u, 0u));
+            }
+            if (lane == 0) cp_async4(raw + 512 * (kCopies + 1), p.scales + j);
+          }
+          ++copied;
+          j0 += G;
+        }
+        cp_async_commit();
+      };
+      auto half8 = [](uint32_t x, uint32_t y) {   // 8 e4m3 -> 8 fp16
+        return make_uint4(e4m3x2_to_f16x2(x), e4m3x2_to_f16x2(x >> 16), e4m3x2_to_f16x2(y), e4m3x2_to_f16x2(y >> 16));
+      };
+#pragma unroll 1
+      for (int d = 0; d < kDepth; ++d) copy_group();
+#pragma unroll 1
+      for (uint32_t gs = 0; gs < copied; ++gs) {
+        const int s = (int)(gs % STAGES);
+        int bad = 0;
+        if (lane == 0 && gs >= (uint32_t)STAGES &&
+            !mbar_wait(empty0 + 8 * s, ((gs / STAGES) + 1) & 1, p.timeout_ns)) {
+          atomicOr(p.err, 4u);
+          bad = 1;
+        }
+        if (__shfl_sync(0xffffffffu, bad, 0)) break;
+        cp_async_wait_group<kDepth - 1>();
+        __syncwarp();   // the slot is free for every lane; lane 0's copy of the scale has landed
+        if ((has >> (gs & 31)) & 1) {
+          const uint32_t slot = smem_u32(smem + (size_t)s * Cfg::kStage);
+          const uint32_t raw = raw0 + (gs % kDepth) * Cfg::kRawGroup + lane * 16;
+          const float sc = ld_shared_f32(raw - lane * 16 + 512 * (kCopies + 1));
+          const uint4 ra = ld_shared_v4(raw);
+          uint4 rb[kCopies];
+#pragma unroll
+          for (int k = 0; k < kCopies; ++k) rb[k] = ld_shared_v4(raw + 512 * (k + 1));
+          // A scale that fp16 holds exactly (any power of two in its range)
+          // multiplies there with the same single rounding as in fp32.
+          if (lane < kARows) {
+            uint4 lo = half8(ra.x, ra.y), hi = half8(ra.z, ra.w);
+            const __half2 sch = __float2half2_rn(sc);
+            const bool exact = __low2float(sch) == sc;
+            uint32_t* h[8] = {&lo.x, &lo.y, &lo.z, &lo.w, &hi.x, &hi.y, &hi.z, &hi.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              __half2 v = *reinterpret_cast<__half2*>(h[k]);
+              if (exact) {
+                v = __hmul2(v, sch);
+              } else {
+                const float2 f = __half22float2(v);
+                v = __floats2half2_rn(f.x * sc, f.y * sc);
+              }
+              *h[k] = *reinterpret_cast<uint32_t*>(&v);
+            }
+            const uint32_t dst = slot + myb * Cfg::kABytes + a_off;
+            st_shared_v4(dst + a_sw, lo);
+            st_shared_v4(dst + (16 ^ a_sw), hi);
+          }
+#pragma unroll
+          for (int k = 0; k < kCopies; ++k) {
+            const uint32_t r7 = (r0 + 2 * k) & 7, ch = (2 * c) & 7;
+            const uint32_t dst = slot + b_off + myb * Cfg::kPanelBytes + k * 256;
+            st_shared_v4(dst + ((ch ^ r7) << 4), half8(rb[k].x, rb[k].y));
+            st_shared_v4(dst + (((ch + 1) ^ r7) << 4), half8(rb[k].z, rb[k].w));
+          }
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full0 + 8 * s);
+        copy_group();
+      }
+      cp_async_wait_all();
+    };
+    if constexpr (CONVERT) {
+      convert_stream();
+      failed = 1;   // (the items have been read)
+    }
     for (uint32_t it = 0; !failed; ++it) {
       int item = -1, start = 0, end = 0, nt = 0, ok = 1;
       if (lane == 0) ok = read_item(it, &item, &start, &end, 4u, &nt) ? 1 : 0;
@@ -762,7 +921,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             failed = true;
             break;
           }
-          if constexpr (GATHER) fence_proxy_async_smem();   // gathered rows are written by threads, not by TMA
+          if constexpr (GATHER || CONVERT) fence_proxy_async_smem();   // written by threads, not by TMA
           tc_fence_after();
           const uint32_t a_slot = smem_u32(smem + (size_t)s * Cfg::kStage);
           const uint32_t b_slot = a_slot + Cfg::kAStage;
@@ -900,7 +1059,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             float v[16];
             if (!empty) {
               tmem_ld16(taddr + c0, v);
-              if constexpr (Cfg::kE4) {
+              if constexpr (Cfg::kE4 || CONVERT) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) v[i] *= p.b_scale;
               }
@@ -960,16 +1119,16 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 using TcFn = void (*)(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap,
                       const CUtensorMap, const CUtensorMap, const TcParams);
 struct TcEntry {
-  int br, mode, nt, stages, acc, group;
-  bool gather;
+  int br, mode, nt, stages, acc, group, feed;
   TcFn fn;
   size_t smem;
   int tmem_cols;
 };
-#define SPMM_TC_ENTRY_AS(BR, NT, ST, MODE, ACC, G, GATHER)                                 \
-  TcEntry{BR, MODE, NT, ST, ACC, G, GATHER, &k_bcsr_tc<BR, NT, ST, MODE, ACC, G, GATHER>,  \
-          TcCfg<BR, NT, ST, MODE, ACC, G>::kSmem, TcCfg<BR, NT, ST, MODE, ACC, G>::kTmemCols}
-#define SPMM_TC_ENTRY(BR, NT, ST, MODE, ACC, G) SPMM_TC_ENTRY_AS(BR, NT, ST, MODE, ACC, G, false)
+#define SPMM_TC_ENTRY_AS(BR, NT, ST, MODE, ACC, G, FEED)                                   \
+  TcEntry{BR, FEED == kFeedConvert ? MODE_E4M3 : MODE, NT, ST, ACC, G, FEED,               \
+          &k_bcsr_tc<BR, NT, ST, MODE, ACC, G, FEED>,                                      \
+          TcCfg<BR, NT, ST, MODE, ACC, G, FEED>::kSmem, TcCfg<BR, NT, ST, MODE, ACC, G, FEED>::kTmemCols}
+#define SPMM_TC_ENTRY(BR, NT, ST, MODE, ACC, G) SPMM_TC_ENTRY_AS(BR, NT, ST, MODE, ACC, G, kFeedTma)
 
 // Instantiated (block height, column tile, ring depth in groups, accumulators,
 // group size) per type.
@@ -992,7 +1151,7 @@ const TcEntry kTcEntries[] = {
     // the planned hybrid product (gather blocks): instances of their own, whose
     // code a plan of 16-row blocks does not carry (7200 x 4096, 5 %, N 1024: 17.9
     // us with it, 17.4 without)
-    SPMM_TC_ENTRY_AS(16, 256, 3, MODE_F16, 2, 4, true), SPMM_TC_ENTRY_AS(16, 512, 3, MODE_F16, 1, 2, true),
+    SPMM_TC_ENTRY_AS(16, 256, 3, MODE_F16, 2, 4, kFeedGather), SPMM_TC_ENTRY_AS(16, 512, 3, MODE_F16, 1, 2, kFeedGather),
     SPMM_TC_ENTRY(64, 256, 2, MODE_SPLIT, 2, 2),
     SPMM_TC_ENTRY(64, 128, 3, MODE_SPLIT, 2, 2),
     SPMM_TC_ENTRY(64, 512, 2, MODE_SPLIT, 1, 1),
@@ -1004,6 +1163,8 @@ const TcEntry kTcEntries[] = {
     SPMM_TC_ENTRY(64, 256, 4, MODE_E4M3, 1, 4), SPMM_TC_ENTRY(64, 512, 4, MODE_E4M3, 1, 4),
     SPMM_TC_ENTRY(32, 256, 4, MODE_E4M3, 1, 4), SPMM_TC_ENTRY(16, 256, 4, MODE_E4M3, 1, 4),
     SPMM_TC_ENTRY(16, 256, 3, MODE_E4M3, 2, 4),
+    // e4m3 converted to fp16: the fp16 kernels' shapes
+    SPMM_TC_ENTRY_AS(64, 256, 3, MODE_F16, 2, 2, kFeedConvert), SPMM_TC_ENTRY_AS(32, 256, 2, MODE_F16, 2, 4, kFeedConvert),
 };
 
 int tc_mode(spmm_dtype d) {
@@ -1014,13 +1175,13 @@ int tc_mode(spmm_dtype d) {
 // The instantiation a request runs on (NULL if none): column tile (default 128
 // for 64-row blocks and N <= 128, else 256), then the first entry matching the
 // requested depth and accumulator count.
-const TcEntry* find_tc(int bR, int mode, int N, const spmm_config& cfg, int* nt_out, bool gather = false) {
+const TcEntry* find_tc(int bR, int mode, int N, const spmm_config& cfg, int* nt_out, int feed = kFeedTma) {
   int nt = cfg.n_tile;
   if (nt <= 0) nt = (N <= 128 && bR == 64) ? 128 : 256;
   if (nt < 256 && bR != 64) nt = 256;
   *nt_out = nt;
   for (const TcEntry& c : kTcEntries) {
-    if (c.br != bR || c.mode != mode || c.nt != nt || c.gather != gather) continue;
+    if (c.br != bR || c.mode != mode || c.nt != nt || c.feed != feed) continue;
     if (cfg.stages > 0 && c.stages != cfg.stages) continue;
     if (cfg.acc_buffers > 0 && c.acc != cfg.acc_buffers) continue;
     return &c;
@@ -1061,7 +1222,8 @@ spmm_status launch_tc(const LaunchRequest& r) {
     return fail(SPMM_ERR_UNSUPPORTED, "the hybrid product and gather blocks run in fp16 / bf16");
   if (e4 && !A.scales) return fail(SPMM_ERR_INVALID_ARG, "E4M3 needs per-block scales");
   int nt = 0;
-  const TcEntry* e = find_tc(A.bR, mode, r.N, r.cfg, &nt, r.gather_rows != nullptr);
+  const TcEntry* e = find_tc(A.bR, mode, r.N, r.cfg, &nt,
+                             r.convert ? kFeedConvert : r.gather_rows ? kFeedGather : kFeedTma);
   if (!e)
     return fail(SPMM_ERR_UNSUPPORTED, "no tcgen05 kernel for bR=" + std::to_string(A.bR) +
                                           " n_tile=" + std::to_string(nt));
@@ -1080,6 +1242,9 @@ spmm_status launch_tc(const LaunchRequest& r) {
                   (r.member_bR != 16 && r.member_bR != 32) || r.stack * r.member_bR != 64))
     return fail(SPMM_ERR_UNSUPPORTED, "a stacked run takes 16- or 32-row fp16 / bf16 blocks on the 64-row pipeline");
   CUtensorMap tmA1, tmAg, tmAlo1, tmAlog, tmB, tmBlo;
+  std::memset(&tmA1, 0, sizeof(tmA1));
+  std::memset(&tmAg, 0, sizeof(tmAg));
+  std::memset(&tmB, 0, sizeof(tmB));
   const void* vals = A.vals ? A.vals : B.data;   // no stored blocks: never dereferenced
   // A's values as a [rows x 16] matrix: 16-bit with 32-byte swizzle (the UMMA
   // K-major SW32 layout), or e4m3 bytes unswizzled (K-major, 8 x 16-byte core
@@ -1089,19 +1254,21 @@ spmm_status launch_tc(const LaunchRequest& r) {
   const uint64_t arow = e4 ? 16 : 32;
   // (a stacked run: A.vals holds the member blocks, bR = member_bR rows each,
   // and the same rows bound: (M / bR) * (K / 16) * bR rows for any bR)
-  spmm_status st = encode_tile_map_2d(&tmA1, adt, vals, 16, rows_bound, arow, 16,
-                                      (uint32_t)(stacked ? r.member_bR : A.bR), aswz);
-  if (st != SPMM_OK) return st;
-  st = encode_tile_map_2d(&tmAg, adt, vals, 16, rows_bound, arow, 16, (uint32_t)(e->group * A.bR), aswz);
-  if (st != SPMM_OK) return st;
+  spmm_status st = SPMM_OK;
+  if (!r.convert) {   // (converted e4m3 is read with plain loads)
+    st = encode_tile_map_2d(&tmA1, adt, vals, 16, rows_bound, arow, 16, (uint32_t)(stacked ? r.member_bR : A.bR), aswz);
+    if (st != SPMM_OK) return st;
+    st = encode_tile_map_2d(&tmAg, adt, vals, 16, rows_bound, arow, 16, (uint32_t)(e->group * A.bR), aswz);
+    if (st != SPMM_OK) return st;
+  }
   // B panels: one 3-D copy per panel when N is a multiple of the 128-byte box
   // width (64 16-bit or 128 e4m3 columns), else one 2-D copy per box.
   const int esz = e4 ? 1 : 2, box_cols = 128 / esz;
-  int panel3d = (r.N % box_cols == 0) ? 1 : 0;
+  int panel3d = (r.N % box_cols == 0 && !r.convert) ? 1 : 0;
   if (panel3d && encode_panel_map_3d(&tmB, B.data, (uint64_t)r.N, (uint64_t)A.K, (uint64_t)B.ldb * esz,
                                      (uint32_t)(nt / box_cols), esz) != SPMM_OK)
     panel3d = 0;
-  if (!panel3d) {
+  if (!panel3d && !r.convert) {
     st = encode_tile_map_2d(&tmB, e4 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16, B.data,
                             (uint64_t)r.N, (uint64_t)A.K, (uint64_t)B.ldb * esz, (uint32_t)box_cols, 16,
                             CU_TENSOR_MAP_SWIZZLE_128B);

@@ -1,0 +1,59 @@
+"""The default e4m3 product at sizes where it runs converted to fp16 on the
+tcgen05 pipeline (spmm_bcsr_mm_nnzb's rule: at least ten blocks a row, as many
+items as CTAs): block scales that fp16 holds and others, part tiles of columns,
+rows of odd block counts, empty rows, rows of more than 32 blocks, a leading
+dimension above N with NaN bytes beyond it.
+
+The reference forms A as the kernel does, round_fp16(e4m3 * scale), and sums in
+FP64. Products of two fp16 are exact in fp32, so a sum of n terms is off by at
+most n steps of 2^-23 of the sum of |a| |b|, and B's scale adds one rounding."""
+import numpy as np
+import pytest
+
+import matrixmultiplicationcuda_gb300 as m
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bR", [32, 64])
+@pytest.mark.parametrize("N,pad,K", [(512, 0, 272), (400, 16, 272), (256, 0, 1040), (768, 0, 256)])
+@pytest.mark.parametrize("scales", ["powers", "any"])
+def test_converted_product(dev, bR, N, pad, K, scales):
+    tiles = -(-N // 256)
+    MB, KB = -(-320 // tiles) + 1, K // 16
+    rng = np.random.default_rng(N + K + bR)
+    keep = rng.uniform(size=(MB, KB)) < 0.9
+    keep[3] = False
+    keep[5, 1:] = False
+    assert keep.sum() >= 10 * MB
+    g = torch.Generator(device=dev).manual_seed(N + bR)
+
+    def e4m3(*shape):
+        v = torch.randint(0, 256, shape, generator=g, device=dev, dtype=torch.uint8)
+        v[(v & 0x7f) == 0x7f] = 0          # no NaN
+        return v
+
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a.astype(np.int32))).to(dev)
+    n = int(keep.sum())
+    vals = e4m3(n, bR, 16)
+    if scales == "powers":                  # down to products that are subnormal in fp16
+        sc = torch.exp2(torch.randint(-12, 3, (n,), generator=g, device=dev).float())
+    else:
+        sc = torch.rand(n, generator=g, device=dev) * 0.02 + 1e-4
+    A = m.BCSR(MB * bR, K, bR, 16, t(np.concatenate([[0], np.cumsum(keep.sum(1))])), t(np.nonzero(keep)[1]),
+               vals.view(-1), m.DType.E4M3, None, sc)
+    Bw = torch.full((K, N + pad), 0x7f, dtype=torch.uint8, device=dev)
+    Bw[:, :N] = e4m3(K, N)
+    C = torch.full((MB * bR, N), float("nan"), device=dev)
+    m.spmm(A, Bw[:, :N], N=N, C=C, b_scale=0.75)
+    m.device_error_check()
+    blocks = (vals.view(torch.float8_e4m3fn).float() * sc[:, None, None]).half().double()
+    Ad = torch.zeros(MB, KB, bR, 16, dtype=torch.float64, device=dev)
+    Ad[torch.from_numpy(keep).to(dev)] = blocks
+    Ad = Ad.permute(0, 2, 1, 3).reshape(MB * bR, K)
+    Bd = Bw[:, :N].contiguous().view(torch.float8_e4m3fn).double()
+    ref = 0.75 * (Ad @ Bd)
+    terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
+    bound = 0.75 * terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs()) + 2.0 ** -24 * ref.abs()
+    assert ((C.double() - ref).abs() <= bound).all()
