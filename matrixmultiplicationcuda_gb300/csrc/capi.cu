@@ -302,7 +302,12 @@ namespace spmm {
 //     2 %, N 512: 30.5 against 33.9 for tc256).
 //   e4m3: mma.sync or, where converts_e4m3 says so, the tcgen05 pipeline with
 //     e4m3 converted to fp16; both take any block scale (the block-scaled MMA,
-//     which a caller may ask for, is faster but needs powers of two).
+//     which a caller may ask for, is faster but needs powers of two). 16 rows and
+//     2048 items or more: mma.sync's 256-column tile (8192^2, 10 %, N 1024: 95
+//     against 119 for 128 columns; 2 % and log-normal rows, N 2048: 58 against 71;
+//     16384 x 4096, 2 %, N 512: 14.8 against 17.5). With fewer, 128 columns
+//     spread long rows further (16384 x 4096, log-normal, N 256: 20.6 against
+//     24.2), as where half of the last 256 would be empty (N 272: 14.1, 14.4).
 spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnzb) {
   spmm_config c;
   std::memset(&c, 0, sizeof(c));
@@ -335,6 +340,8 @@ spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnz
   }
   c.kernel = 1;
   c.n_tile = bR == 64 && dtype != SPMM_E4M3 && dtype != SPMM_F16_SPLIT ? 64 : mma_default_nt(bR, dtype, N);
+  if (dtype == SPMM_E4M3 && bR == 16 && N > 128 && (N <= 256 || N > 384) && (long long)(M / 16) * ((N + 255) / 256) >= 2048)
+    c.n_tile = 256;
   c.stages = 4;
   return c;
 }

@@ -57,3 +57,31 @@ def test_converted_product(dev, bR, N, pad, K, scales):
     terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
     bound = 0.75 * terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs()) + 2.0 ** -24 * ref.abs()
     assert ((C.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("N", [144, 256, 400])
+def test_sixteen_rows_many_items(dev, N):
+    """16-row blocks with at least 2048 items of 256 columns (mma.sync's wider
+    tile), empty rows and part tiles; products and bound as above."""
+    MB, K, bR = -(-2048 // -(-N // 256)), 160, 16
+    rng = np.random.default_rng(N)
+    keep = rng.uniform(size=(MB, K // 16)) < 0.4
+    keep[::7] = False
+    g = torch.Generator(device=dev).manual_seed(N)
+    n = int(keep.sum())
+    vals = torch.randint(0, 0x7f, (n, bR, 16), generator=g, device=dev, dtype=torch.uint8)
+    sc = torch.rand(n, generator=g, device=dev) * 0.02 + 1e-4
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a.astype(np.int32))).to(dev)
+    A = m.BCSR(MB * bR, K, bR, 16, t(np.concatenate([[0], np.cumsum(keep.sum(1))])), t(np.nonzero(keep)[1]),
+               vals.view(-1), m.DType.E4M3, None, sc)
+    B = torch.randint(0, 0x7f, (K, N), generator=g, device=dev, dtype=torch.uint8)
+    C = torch.full((MB * bR, N), float("nan"), device=dev)
+    m.spmm(A, B, C=C)
+    m.device_error_check()
+    Ad = torch.zeros(MB, K // 16, bR, 16, dtype=torch.float64, device=dev)
+    Ad[torch.from_numpy(keep).to(dev)] = (vals.view(torch.float8_e4m3fn).float() * sc[:, None, None]).half().double()
+    Ad = Ad.permute(0, 2, 1, 3).reshape(MB * bR, K)
+    Bd = B.view(torch.float8_e4m3fn).double()
+    terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
+    bound = terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs())
+    assert ((C.double() - Ad @ Bd).abs() <= bound).all()
