@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(128) k_mlp_reduce(const __grid_constant__ Redu
   }
   __syncthreads();
   const double total = tot[1] > 0 ? tot[1] : 1.0;
-  if (is_w || is_b) p.grad[L.gw + k] = (float)(2.0 / total) * s;
+  if (is_w || is_b) p.grad[L.gw + k] = (float)(2.0 / total * s);   // the factor rounds once, with the product
   if (l == 0 && k < 2 * p.s.in) p.grad[k] = 0.f;
   if (l == 0 && k == 0 && p.loss) *p.loss = (float)(tot[0] / total);
 }
