@@ -293,9 +293,10 @@ spmm_status spmm_batch_plan_info(const spmm_batch_plan* plan, int* items, int* s
 spmm_status spmm_batch_plan_destroy(spmm_batch_plan* plan);
 
 /* ---- hybrid BCSR + CSR (HCSRMatrix, formats/HCSRMatrix.cpp:10-36) -------------
- * C = A_blocks B + A_rest B in ONE launch: the tcgen05 pipeline multiplies the
- * BCSR part (any block height; the reference uses 16 x 16), and its epilogue
- * warps add the CSR part's entries to each tile after storing it. The reference
+ * C = A_blocks B + A_rest B: the tcgen05 pipeline multiplies the BCSR part (any
+ * block height; the reference uses 16 x 16). The CSR part's entries are added to
+ * C by a second launch or, for small C and with a cfg, by the pipeline's
+ * epilogue warps, tile by tile after they stored it. The reference
  * runs three kernels (CSR into a second buffer, BCSR into C, then an
  * element-wise add; main.cu:567-590). fp16 only, no split-K. Both parts
  * describe the same M x K matrix; A_rest->row_ptr has M + 1 entries, col_idx

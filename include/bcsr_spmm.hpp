@@ -69,7 +69,7 @@ class BCSRMatrix {
 // HCSRMatrix(matrix, threshold) (formats/HCSRMatrix.cpp:10-36): the 16x16
 // blocks whose density (nonzero elements / 256) is >= threshold form a 16x16
 // BCSR part, every other element a CSR part. spmm_hcsr_mm multiplies both
-// parts in one launch.
+// parts into one C.
 class HCSRMatrix {
  public:
   BCSRMatrix* bcsr = nullptr;

@@ -88,9 +88,10 @@ def spmm(A: BCSR, B, N=None, C=None, cfg: Optional[Config] = None, stream=None, 
 
 def hcsr_mm(A_blocks: BCSR, csr_row_ptr, csr_col_idx, csr_vals, B, N=None, C=None,
             cfg: Optional[Config] = None, stream=None, ldc=None):
-    """Hybrid product C = A_blocks @ B + A_rest @ B in one launch (fp16): the
-    BCSR part on the tensor cores, the CSR part (row_ptr [M+1], col_idx, fp16
-    vals, device tensors) added in the same kernel's epilogue."""
+    """Hybrid product C = A_blocks @ B + A_rest @ B (fp16): the BCSR part on the
+    tensor cores, the CSR part (row_ptr [M+1], col_idx, fp16 vals, device
+    tensors) added to C by a second launch or, for small products and with a
+    cfg, in the same kernel's epilogue."""
     torch = _torch()
     N = int(B.shape[1]) if N is None else int(N)
     if C is None:

@@ -22,33 +22,45 @@ __device__ __forceinline__ void fma8(float (&acc)[8], float a, uint4 b) {
 }
 
 // acc[0..7] += sum over entries e in [e0, e1) of vals[e] * B[col_idx[e]][n..n+7],
-// U entries' B loads in flight. Warp-uniform e0 / e1 (every lane reads the same
-// entry, one broadcast load); `valid` (this lane's columns lie inside B) may
-// differ per lane.
+// in order, U entries' B loads in flight. Warp-uniform e0 / e1; `valid` (this
+// lane's columns lie inside B) may differ per lane. Lanes read 32 entries'
+// indices and values together, 32 entries ahead of their use, so that a B load
+// waits for no index, and the last entries of a row load together like any
+// others (one by one, with their indices read first, a row's last U - 1 entries
+// took as long as 2 U (U - 1) others).
 template <int U>
 __device__ __forceinline__ void csr_row_slice(const int* __restrict__ col_idx, const __half* __restrict__ vals,
                                               const __half* __restrict__ B, long long ldb, int e0, int e1, int n,
                                               bool valid, float (&acc)[8]) {
-  int e = e0;
-  for (; e + U <= e1; e += U) {
-    int k[U];
-    float a[U];
-    uint4 b[U];
-#pragma unroll
-    for (int t = 0; t < U; ++t) {
-      k[t] = __ldg(col_idx + e + t);
-      a[t] = __half2float(vals[e + t]);
-    }
-#pragma unroll
-    for (int t = 0; t < U; ++t)
-      b[t] = valid ? __ldg(reinterpret_cast<const uint4*>(B + (long long)k[t] * ldb + n)) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-    for (int t = 0; t < U; ++t) fma8(acc, a[t], b[t]);
+  const int lane = threadIdx.x & 31;
+  const __half* src = B + (valid ? n : 0);
+  int next_k = 0;
+  __half next_a = __float2half(0.f);
+  if (e0 + lane < e1) {
+    next_k = __ldg(col_idx + e0 + lane);
+    next_a = __ldg(vals + e0 + lane);
   }
-  for (; e < e1; ++e) {
-    const int k = __ldg(col_idx + e);
-    const float a = __half2float(vals[e]);
-    if (valid) fma8(acc, a, __ldg(reinterpret_cast<const uint4*>(B + (long long)k * ldb + n)));
+  for (int base = e0; base < e1; base += 32) {
+    const int cnt = min(32, e1 - base), ks = next_k;
+    const float as = __half2float(next_a);
+    if (base + 32 + lane < e1) {
+      next_k = __ldg(col_idx + base + 32 + lane);
+      next_a = __ldg(vals + base + 32 + lane);
+    }
+    for (int i = 0; i < cnt; i += U) {
+      // (no condition on a load: past the last entry its row again, past N column 0)
+      uint4 b[U];
+#pragma unroll
+      for (int t = 0; t < U; ++t) {
+        const unsigned k = (unsigned)__shfl_sync(0xffffffffu, ks, min(i + t, cnt - 1));
+        b[t] = __ldg(reinterpret_cast<const uint4*>(src + (unsigned long long)k * (unsigned)ldb));
+      }
+#pragma unroll
+      for (int t = 0; t < U; ++t) {
+        const float a = __shfl_sync(0xffffffffu, as, (i + t) & 31);
+        if (i + t < cnt) fma8(acc, a, b[t]);
+      }
+    }
   }
 }
 

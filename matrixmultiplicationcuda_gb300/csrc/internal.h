@@ -102,6 +102,9 @@ struct LaunchRequest {
 // The tcgen05 pipeline's column tile and CTAs per SM for a product (false when
 // it has no kernel for it): what a plan builds its item list for.
 bool tc_geometry(int bR, spmm_dtype dtype, int N, const spmm_config& cfg, int* nt, int* ctas_per_sm);
+// C += A B for a CSR matrix (csr.cu)
+spmm_status launch_csr_add(const spmm_csr_desc& A, const spmm_dense_desc& B, int N, float* C, long long ldc,
+                           cudaStream_t stream);
 // mma.sync family (spmm_mma.cu)
 spmm_status launch_mma(const LaunchRequest& r);
 // tcgen05 family (spmm_tc.cu); returns SPMM_ERR_UNSUPPORTED when it has no kernel for r

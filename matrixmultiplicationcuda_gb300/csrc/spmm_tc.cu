@@ -108,8 +108,10 @@ __device__ __forceinline__ void st_release_gpu(unsigned* ptr, unsigned v) {
 }
 
 // Who writes a group's slot: TMA alone; the planned hybrid product's gather
-// blocks (B rows copied by the B issuers); e4m3 converted to fp16 by them.
-enum Feed : int { kFeedTma = 0, kFeedGather = 1, kFeedConvert = 2 };
+// blocks (B rows copied by the B issuers); e4m3 converted to fp16 by them. The
+// hybrid product's CSR pass is an instance of its own too, so that no other
+// epilogue shares its registers with it.
+enum Feed : int { kFeedTma = 0, kFeedGather = 1, kFeedConvert = 2, kFeedCsr = 3 };
 
 // BR: block height (the UMMA N); NT: output columns per item; STAGES: ring
 // depth in groups; ACC: TMEM accumulators per CTA (2 = one item's epilogue
@@ -798,7 +800,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
                   // an SM, one TMA copies 161; shared memory alone takes 128 of either
                   // (8 KB written, then read by the MMAs).
                   uint8_t* b_dst = b_dst0 + (size_t)b * Cfg::kPanelBytes;
-                  const bool whole = __all_sync(0xffffffffu, lane >= 16 || rows < p.K);
+                  const bool whole = __all_sync(0xffffffffu, lane >= 16 || (unsigned)rows < (unsigned)p.K);
 #pragma unroll
                   for (int c0 = 0; c0 < NT / 8; c0 += 32) {
                     // this lane's 8 columns of each row (past N: any columns, their results go nowhere)
@@ -814,8 +816,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
                     } else {
                       for (int r = 0; r < 16; ++r) {
                         const int row = __shfl_sync(0xffffffffu, rows, r);
-                        cp_async16_or_zero(dst + r * 128 + (sw ^ ((r & 7) << 4)),
-                                           src + (row < p.K ? (long long)row * p.ldb : 0), row < p.K);
+                        const bool in = (unsigned)row < (unsigned)p.K;   // (an index outside A reads zeros too)
+                        cp_async16_or_zero(dst + r * 128 + (sw ^ ((r & 7) << 4)), src + (in ? (long long)row * p.ldb : 0),
+                                           in);
                       }
                     }
                   }
@@ -975,7 +978,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   } else if (warp >= 4 && warp < 8) {
     // ------------------------------ epilogue (warps 4-7) ---------------------------
     const int q4 = warp & 3;                // TMEM lane quarter this warp may access
-    const bool hybrid = p.csr_row_ptr != nullptr;
+    constexpr bool hybrid = FEED == kFeedCsr;
     const bool planned = p.pair != nullptr;
     for (uint32_t it = 0;; ++it) {
       int item = -1, start = 0, end = 0, ok = 1;
@@ -1137,17 +1140,18 @@ struct TcEntry {
 // KB of shared memory per SM): the pipeline is bound by the latency of its
 // copies, and the fifth group measured ~2 % faster than four on the headline
 // product.
-#define SPMM_TC_SHAPES(MODE)                                                                         \
-  SPMM_TC_ENTRY(64, 256, 5, MODE, 2, 2), SPMM_TC_ENTRY(64, 256, 4, MODE, 2, 2),                     \
-      SPMM_TC_ENTRY(64, 256, 2, MODE, 2, 4),                                                        \
-      SPMM_TC_ENTRY(64, 512, 3, MODE, 1, 2), SPMM_TC_ENTRY(64, 512, 3, MODE, 2, 4),                 \
-      SPMM_TC_ENTRY(64, 128, 4, MODE, 2, 4), SPMM_TC_ENTRY(32, 256, 3, MODE, 2, 4),                 \
-      SPMM_TC_ENTRY(32, 512, 3, MODE, 1, 2), SPMM_TC_ENTRY(16, 256, 3, MODE, 2, 4),                 \
-      SPMM_TC_ENTRY(16, 512, 3, MODE, 1, 2)
+#define SPMM_TC_SHAPES(MODE, FEED)                                                                         \
+  SPMM_TC_ENTRY_AS(64, 256, 5, MODE, 2, 2, FEED), SPMM_TC_ENTRY_AS(64, 256, 4, MODE, 2, 2, FEED),                     \
+      SPMM_TC_ENTRY_AS(64, 256, 2, MODE, 2, 4, FEED),                                                        \
+      SPMM_TC_ENTRY_AS(64, 512, 3, MODE, 1, 2, FEED), SPMM_TC_ENTRY_AS(64, 512, 3, MODE, 2, 4, FEED),                 \
+      SPMM_TC_ENTRY_AS(64, 128, 4, MODE, 2, 4, FEED), SPMM_TC_ENTRY_AS(32, 256, 3, MODE, 2, 4, FEED),                 \
+      SPMM_TC_ENTRY_AS(32, 512, 3, MODE, 1, 2, FEED), SPMM_TC_ENTRY_AS(16, 256, 3, MODE, 2, 4, FEED),                 \
+      SPMM_TC_ENTRY_AS(16, 512, 3, MODE, 1, 2, FEED)
 
 const TcEntry kTcEntries[] = {
-    SPMM_TC_SHAPES(MODE_F16),
-    SPMM_TC_SHAPES(MODE_BF16),
+    SPMM_TC_SHAPES(MODE_F16, kFeedTma),
+    SPMM_TC_SHAPES(MODE_BF16, kFeedTma),
+    SPMM_TC_SHAPES(MODE_F16, kFeedCsr),
     // the planned hybrid product (gather blocks): instances of their own, whose
     // code a plan of 16-row blocks does not carry (7200 x 4096, 5 %, N 1024: 17.9
     // us with it, 17.4 without)
@@ -1223,7 +1227,7 @@ spmm_status launch_tc(const LaunchRequest& r) {
   if (e4 && !A.scales) return fail(SPMM_ERR_INVALID_ARG, "E4M3 needs per-block scales");
   int nt = 0;
   const TcEntry* e = find_tc(A.bR, mode, r.N, r.cfg, &nt,
-                             r.convert ? kFeedConvert : r.gather_rows ? kFeedGather : kFeedTma);
+                             r.convert ? kFeedConvert : r.gather_rows ? kFeedGather : r.csr ? kFeedCsr : kFeedTma);
   if (!e)
     return fail(SPMM_ERR_UNSUPPORTED, "no tcgen05 kernel for bR=" + std::to_string(A.bR) +
                                           " n_tile=" + std::to_string(nt));
