@@ -297,7 +297,17 @@ namespace spmm {
 //     (41 blocks a row), N 512: 18.2 against 28.8; 1 % (5 a row): 8.8 against
 //     8.5. 16 rows, 8 %: 26.5 against 30.4; 1 %: 11.5 against 9.2; 8192^2 with
 //     log-normal rows, 8 %: 51 against 123. Its column tile is 256 wide, so
-//     narrower products stay.
+//     narrower products stay. With many items, so that its CTAs have a next one
+//     to overlap, it pays on shorter rows: 32 rows, 2 % (10 a row), N 1024: 17.0
+//     against 22.0, 5.7 a row 14.4, 16.6, log-normal, 1.2 %, N 512: 10.2, 12.8;
+//     16 rows, 10 a row, N 1024: 20.9, 22.0, log-normal, 15 a row, N 2048: 50, 63.
+//     On mma.sync, rows of six blocks and more take the ring of eight (a group
+//     of four in the time of two blocks, the 16-row tile of 256 columns only
+//     where its three CTAs per SM hold all items): 2048^2 log-normal, 16 rows, 6.6
+//     a row, N 512: 9.8 -> 7.2, 8192^2, N 104: 24.1 -> 18.7; the 256-column tile
+//     with more items: 8192^2, 6 a row, N 512: 9.7 against 10.2 with the larger
+//     ring. 64 columns or fewer then take the 128-column tile (4096^2, 12.7 a row:
+//     5.3 against 6.6) unless there are block rows enough (16384: 8.1, 7.9).
 //   split fp16, 64-row blocks above 128 columns: the 64-row pipeline (16384^2,
 //     2 %, N 512: 30.5 against 33.9 for tc256).
 //   e4m3: mma.sync or, where converts_e4m3 says so, the tcgen05 pipeline with
@@ -333,8 +343,12 @@ spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnz
         tc(2, 256, 2);
       else if (nnzb < 0 || nnzb > 100)
         tc(3, 256, 0);
-    } else if (dtype != SPMM_F16_SPLIT && N > 128 && row >= (bR == 16 ? 16 : 12)) {
-      tc(2, 256, 2);
+    } else if (dtype != SPMM_F16_SPLIT && N > 128) {
+      const long long items = (long long)(M / bR) * ((N + 255) / 256);
+      const bool whole = N <= 256 || N > 384;   // the last 256-column tile at least half used
+      if (row >= (bR == 16 ? 16 : 12) ||
+          (whole && (bR == 16 ? row >= 10 && items >= 1024 : row >= 5 && items >= 3ll * sm_count())))
+        tc(2, 256, 2);
     }
     if (c.kernel != 0) return c;
   }
@@ -343,6 +357,10 @@ spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnz
   if (dtype == SPMM_E4M3 && bR == 16 && N > 128 && (N <= 256 || N > 384) && (long long)(M / 16) * ((N + 255) / 256) >= 2048)
     c.n_tile = 256;
   c.stages = 4;
+  if (bR != 64 && (dtype == SPMM_F16 || dtype == SPMM_BF16) && row >= 5.5) {
+    if (c.n_tile == 64 && (N > 64 || M / bR < 4 * sm_count())) c.n_tile = 128;
+    if (c.n_tile == 128 || (c.n_tile == 256 && (M / 16) * ((N + 255ll) / 256) <= 3 * sm_count())) c.stages = 8;
+  }
   return c;
 }
 

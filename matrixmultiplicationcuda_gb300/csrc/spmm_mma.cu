@@ -18,17 +18,29 @@ struct Entry {
   int threads;
 };
 
-#define SPMM_MMA_ENTRY(BR, NT, WM, WN, ST, MODE)                                   \
+#define SPMM_MMA_ENTRY_AS(BR, NT, WM, WN, ST, RING, GROUP, MODE)                   \
   Entry{BR,                                                                        \
         MODE,                                                                      \
         NT,                                                                        \
         ST,                                                                        \
         WM,                                                                        \
         WN,                                                                        \
-        &k_bcsr_mma<BR, NT, WM, WN, ST, MODE>,                                     \
-        MmaCfg<BR, NT, WM, WN, ST, MODE>::kSmem,                                   \
-        MmaCfg<BR, NT, WM, WN, ST, MODE>::kThreads}
+        &k_bcsr_mma<BR, NT, WM, WN, RING, GROUP, MODE>,                            \
+        MmaCfg<BR, NT, WM, WN, RING, GROUP, MODE>::kSmem,                          \
+        MmaCfg<BR, NT, WM, WN, RING, GROUP, MODE>::kThreads}
+#define SPMM_MMA_ENTRY(BR, NT, WM, WN, ST, MODE) \
+  SPMM_MMA_ENTRY_AS(BR, NT, WM, WN, ST, ST, (ST >= 8 ? 4 : 1), MODE)
 
+// A ring of eight blocks takes them in two groups of four: the producer waits,
+// expects bytes and copies A's blocks (contiguous) once per group, and the
+// consumers wait and arrive once, so a row's next block follows after ~110 ns
+// instead of ~215, which is what long rows are bound by (16 rows, log-normal,
+// 8192^2, 2 % (up to 95 blocks a row), N 128: 21.8 us with single blocks, 14.7;
+// even rows of 10: 7.1 and 6.4). A ring of four keeps single blocks: rows shorter
+// than a group leave part of its slots empty (two blocks a row, 16384 x 2048, N
+// 1024: 16.1 us, 16.8 with groups). e4m3's blocks are half as large, so its
+// rings hold eight at the same occupancy (16 rows, 8192^2, 10 %, N 1024: 119
+// us with single blocks, 102; log-normal rows, 5 %, N 512: 77, 58).
 // The configuration space the tuner sweeps (block height x column tile x depth).
 #define SPMM_MMA_SHAPES(MODE)                                                      \
   SPMM_MMA_ENTRY(16, 64, 1, 4, 4, MODE), SPMM_MMA_ENTRY(16, 128, 1, 4, 4, MODE),    \
@@ -46,11 +58,11 @@ const Entry kEntries[] = {
     SPMM_MMA_ENTRY(32, 128, 2, 2, 4, MODE_SPLIT),
     SPMM_MMA_ENTRY(64, 128, 2, 2, 4, MODE_SPLIT),
     SPMM_MMA_ENTRY(64, 64, 4, 1, 4, MODE_SPLIT),
-    SPMM_MMA_ENTRY(16, 128, 1, 4, 4, MODE_E4M3),
-    SPMM_MMA_ENTRY(16, 256, 1, 4, 4, MODE_E4M3),
-    SPMM_MMA_ENTRY(32, 128, 2, 2, 4, MODE_E4M3),
-    SPMM_MMA_ENTRY(64, 128, 2, 2, 4, MODE_E4M3),
-    SPMM_MMA_ENTRY(64, 256, 2, 2, 4, MODE_E4M3),
+    SPMM_MMA_ENTRY_AS(16, 128, 1, 4, 4, 8, 4, MODE_E4M3),
+    SPMM_MMA_ENTRY_AS(16, 256, 1, 4, 4, 8, 4, MODE_E4M3),
+    SPMM_MMA_ENTRY_AS(32, 128, 2, 2, 4, 8, 4, MODE_E4M3),
+    SPMM_MMA_ENTRY_AS(64, 128, 2, 2, 4, 8, 4, MODE_E4M3),
+    SPMM_MMA_ENTRY_AS(64, 256, 2, 2, 4, 8, 4, MODE_E4M3),
 };
 
 int mode_of(spmm_dtype d) {

@@ -5,8 +5,10 @@
 // output columns). Within a CTA one producer warp streams, for every stored
 // block of the item's block row, the A block (one untiled TMA bulk copy of its
 // contiguous bR x 16 values) and the matching B row-panel (the 16 rows of B
-// selected by col_idx, NT columns, as 128-byte-swizzled TMA tiles) into a
-// STAGES-deep mbarrier ring. WM x WN consumer warps read fragments with
+// selected by col_idx, NT columns, as 128-byte-swizzled TMA tiles) into an
+// mbarrier ring of STAGES blocks, whose slots hold GROUP consecutive blocks of a
+// row (one wait, one expected byte count and one copy of A for all of them, since
+// the producer's ~400 cycles a block are what bounds a long row). WM x WN consumer warps read fragments with
 // ldmatrix and accumulate in fp32 registers, then write their part of C with
 // streaming stores. The producer runs ahead across item boundaries, so one
 // item's epilogue overlaps the next item's loads.
@@ -43,7 +45,7 @@ struct MmaParams {
   int panel3d;     // 16-bit B panel loaded by one 3-D copy (N % 64 == 0)
 };
 
-template <int BR, int NT, int WM, int WN, int STAGES, int MODE>
+template <int BR, int NT, int WM, int WN, int STAGES, int GROUP, int MODE>
 struct MmaCfg {
   static constexpr int kConsumerWarps = WM * WN;
   static constexpr int kThreads = (kConsumerWarps + 1) * 32;
@@ -58,7 +60,9 @@ struct MmaCfg {
   static constexpr int kParts = kSplit ? 2 : 1;            // hi (+ lo)
   static constexpr int kStageB = kPanelBytes * kParts;      // multiple of 1024
   static constexpr int kStageA = kABytes * kParts;
-  static constexpr int kTxBytes = kStageB + kStageA;
+  // a ring of STAGES blocks, in slots of up to GROUP consecutive blocks of one block row
+  static constexpr int kSlots = STAGES / GROUP;
+  static constexpr int kTxBytes = kStageB + kStageA;   // per block
   static constexpr int kWTM = BR / WM;                      // warp tile rows
   static constexpr int kWTN = NT / WN;                      // warp tile cols
   static constexpr int kMT = kWTM / 16;
@@ -71,22 +75,23 @@ struct MmaCfg {
   static_assert(kABytes % 16 == 0, "bulk copy granularity");
 };
 
-template <int BR, int NT, int WM, int WN, int STAGES, int MODE>
-__global__ void __launch_bounds__(MmaCfg<BR, NT, WM, WN, STAGES, MODE>::kThreads, 1)
+template <int BR, int NT, int WM, int WN, int STAGES, int GROUP, int MODE>
+__global__ void __launch_bounds__(MmaCfg<BR, NT, WM, WN, STAGES, GROUP, MODE>::kThreads, 1)
     k_bcsr_mma(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmBlo,
                const MmaParams p) {
-  using Cfg = MmaCfg<BR, NT, WM, WN, STAGES, MODE>;
+  using Cfg = MmaCfg<BR, NT, WM, WN, STAGES, GROUP, MODE>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~uintptr_t(1023));
   uint8_t* sB = smem;                                         // STAGES x kStageB
   uint8_t* sA = smem + (size_t)STAGES * Cfg::kStageB;         // STAGES x kStageA
   uint64_t* bars = reinterpret_cast<uint64_t*>(sA + (size_t)STAGES * Cfg::kStageA);
-  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
+  constexpr int G = GROUP, SLOTS = Cfg::kSlots;
+  const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + SLOTS);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < SLOTS; ++s) {
       mbar_init(full0 + 8 * s, 1);
       mbar_init(empty0 + 8 * s, Cfg::kConsumerWarps);
     }
@@ -101,7 +106,7 @@ __global__ void __launch_bounds__(MmaCfg<BR, NT, WM, WN, STAGES, MODE>::kThreads
     // Lane 0 issues every copy; the other lanes stage column indices 32 at a time
     // in shared memory and prefetch the next item's row range, so the issuing
     // lane never waits on a global load or a shuffle between two blocks.
-    int* s_cols = reinterpret_cast<int*>(bars + 2 * STAGES);
+    int* s_cols = reinterpret_cast<int*>(bars + 2 * SLOTS);
     if (lane == 0) {
       tma_prefetch_desc(&tmB);
       if (Cfg::kSplit) tma_prefetch_desc(&tmBlo);
@@ -130,35 +135,42 @@ __global__ void __launch_bounds__(MmaCfg<BR, NT, WM, WN, STAGES, MODE>::kThreads
         const int nn = more ? end : nend;
         mycol = (lane < nn - nb && (more || nitem < p.n_items)) ? __ldg(p.col_idx + nb + lane) : 0;
         if (lane == 0) {
-          for (int i = 0; i < cnt; ++i, ++g) {
-            const int s = (int)(g % STAGES);
-            if (g >= (uint32_t)STAGES &&
-                !mbar_wait(empty0 + 8 * s, ((g / STAGES) + 1) & 1, p.timeout_ns)) {
+          for (int i0 = 0; i0 < cnt; i0 += G, ++g) {
+            const int s = (int)(g % SLOTS), n = G == 1 ? 1 : min(G, cnt - i0);
+            if (g >= (uint32_t)SLOTS && !mbar_wait(empty0 + 8 * s, ((g / SLOTS) + 1) & 1, p.timeout_ns)) {
               atomicOr(p.err, 2u);
               failed = 1;
               break;
             }
-            const int col = s_cols[i];
-            const uint32_t fb = full0 + 8 * s;
-            mbar_arrive_expect_tx(fb, Cfg::kTxBytes);
-            const size_t aoff = (size_t)(base + i) * Cfg::kABytes;
-            uint8_t* a_dst = sA + (size_t)s * Cfg::kStageA;
-            tma_bulk_g2s(smem_u32(a_dst), p.vals + aoff, Cfg::kABytes, fb, pol_a);
-            if (Cfg::kSplit)
-              tma_bulk_g2s(smem_u32(a_dst + Cfg::kABytes), p.vals_lo + aoff, Cfg::kABytes, fb, pol_a);
-            uint8_t* b_dst = sB + (size_t)s * Cfg::kStageB;
-            if (MODE != MODE_E4M3 && p.panel3d) {
-              tma_tile_3d_g2s(smem_u32(b_dst), &tmB, 0, col * 16, nt * Cfg::kNBox, fb, pol_b);
-              if (Cfg::kSplit)
-                tma_tile_3d_g2s(smem_u32(b_dst + Cfg::kPanelBytes), &tmBlo, 0, col * 16, nt * Cfg::kNBox, fb, pol_b);
-            } else {
+            int cols[G];   // (read ahead of the copies, which the compiler does not move loads across)
 #pragma unroll
-              for (int b = 0; b < Cfg::kNBox; ++b) {
-                tma_tile_2d_g2s(smem_u32(b_dst + b * Cfg::kBoxBytes), &tmB,
-                                nt * NT + b * Cfg::kBoxCols, col * 16, fb, pol_b);
+            for (int t = 0; t < G; ++t) cols[t] = s_cols[i0 + t];
+            const uint32_t fb = full0 + 8 * s;
+            mbar_arrive_expect_tx(fb, (uint32_t)(n * Cfg::kTxBytes));
+            // the group's A blocks are contiguous, its parts (hi, lo) one after the other
+            const size_t aoff = (size_t)(base + i0) * Cfg::kABytes;
+            uint8_t* a_dst = sA + (size_t)s * G * Cfg::kStageA;
+            tma_bulk_g2s(smem_u32(a_dst), p.vals + aoff, (uint32_t)(n * Cfg::kABytes), fb, pol_a);
+            if (Cfg::kSplit)
+              tma_bulk_g2s(smem_u32(a_dst + G * Cfg::kABytes), p.vals_lo + aoff, (uint32_t)(n * Cfg::kABytes), fb, pol_a);
+#pragma unroll
+            for (int t = 0; t < G; ++t) {
+              if (t >= n) break;
+              const int col = cols[t];
+              uint8_t* b_dst = sB + (size_t)(s * G + t) * Cfg::kStageB;
+              if (MODE != MODE_E4M3 && p.panel3d) {
+                tma_tile_3d_g2s(smem_u32(b_dst), &tmB, 0, col * 16, nt * Cfg::kNBox, fb, pol_b);
                 if (Cfg::kSplit)
-                  tma_tile_2d_g2s(smem_u32(b_dst + Cfg::kPanelBytes + b * Cfg::kBoxBytes), &tmBlo,
+                  tma_tile_3d_g2s(smem_u32(b_dst + Cfg::kPanelBytes), &tmBlo, 0, col * 16, nt * Cfg::kNBox, fb, pol_b);
+              } else {
+#pragma unroll
+                for (int b = 0; b < Cfg::kNBox; ++b) {
+                  tma_tile_2d_g2s(smem_u32(b_dst + b * Cfg::kBoxBytes), &tmB,
                                   nt * NT + b * Cfg::kBoxCols, col * 16, fb, pol_b);
+                  if (Cfg::kSplit)
+                    tma_tile_2d_g2s(smem_u32(b_dst + Cfg::kPanelBytes + b * Cfg::kBoxBytes), &tmBlo,
+                                    nt * NT + b * Cfg::kBoxCols, col * 16, fb, pol_b);
+                }
               }
             }
           }
@@ -190,14 +202,17 @@ __global__ void __launch_bounds__(MmaCfg<BR, NT, WM, WN, STAGES, MODE>::kThreads
 #pragma unroll
         for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.f;
 
-    for (int k = start; k < end; ++k, ++g) {
-      const int s = (int)(g % STAGES);
-      if (!mbar_wait(full0 + 8 * s, (g / STAGES) & 1, p.timeout_ns)) {
+    for (int k0 = start; k0 < end; k0 += G, ++g) {
+      const int s = (int)(g % SLOTS), n = G == 1 ? 1 : min(G, end - k0);
+      if (!mbar_wait(full0 + 8 * s, (g / SLOTS) & 1, p.timeout_ns)) {
         if (lane == 0) atomicOr(p.err, 1u);
         return;
       }
-      const uint32_t a_base = smem_u32(sA + (size_t)s * Cfg::kStageA);
-      const uint32_t b_base = smem_u32(sB + (size_t)s * Cfg::kStageB);
+#pragma unroll 1
+      for (int t = 0; t < n; ++t) {
+      [[maybe_unused]] const int k = k0 + t;
+      const uint32_t a_base = smem_u32(sA + (size_t)s * G * Cfg::kStageA) + t * Cfg::kABytes;
+      const uint32_t b_base = smem_u32(sB + (size_t)(s * G + t) * Cfg::kStageB);
       if constexpr (MODE != MODE_E4M3) {
         // A fragments: rows wm*WTM + mt*16 .. +15, the block's 32-byte rows.
         uint32_t af[Cfg::kParts][Cfg::kMT][4];
@@ -206,7 +221,7 @@ __global__ void __launch_bounds__(MmaCfg<BR, NT, WM, WN, STAGES, MODE>::kThreads
 #pragma unroll
           for (int mt = 0; mt < Cfg::kMT; ++mt) {
             const int row = wm * Cfg::kWTM + mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-            ldsm_x4(a_base + part * Cfg::kABytes + row * 32 + (lane >> 4) * 16, af[part][mt][0],
+            ldsm_x4(a_base + part * G * Cfg::kABytes + row * 32 + (lane >> 4) * 16, af[part][mt][0],
                     af[part][mt][1], af[part][mt][2], af[part][mt][3]);
           }
 #pragma unroll
@@ -243,7 +258,7 @@ __global__ void __launch_bounds__(MmaCfg<BR, NT, WM, WN, STAGES, MODE>::kThreads
 #pragma unroll
         for (int mt = 0; mt < Cfg::kMT; ++mt) {
           const int r0 = wm * Cfg::kWTM + mt * 16 + gq;
-          const uint8_t* a8 = sA + (size_t)s * Cfg::kStageA;
+          const uint8_t* a8 = sA + (size_t)s * G * Cfg::kStageA + t * Cfg::kABytes;
           const uint32_t v[4] = {*reinterpret_cast<const uint16_t*>(a8 + r0 * 16 + 2 * tq),
                                  *reinterpret_cast<const uint16_t*>(a8 + (r0 + 8) * 16 + 2 * tq),
                                  *reinterpret_cast<const uint16_t*>(a8 + r0 * 16 + 2 * tq + 8),
@@ -278,6 +293,7 @@ __global__ void __launch_bounds__(MmaCfg<BR, NT, WM, WN, STAGES, MODE>::kThreads
             }
           }
         }
+      }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(empty0 + 8 * s);

@@ -41,6 +41,11 @@ SHAPES = [(512, 256, 264, 16, 0.3), (512, 512, 264, 16, 0.9), (1024, 512, 136, 3
           (1024, 512, 264, 64, 0.15), (1024, 512, 264, 64, 0.8), (64, 64, 40, 64, 0.9), (8192, 64, 1040, 64, 0.7)]
 
 
+# mma.sync's ring of eight (256-, 128-column tiles, few columns), and tcgen05 for many items
+SHAPES += [(512, 512, 264, 16, 0.3), (512, 512, 136, 16, 0.25), (496, 512, 40, 16, 0.4), (512, 1040, 72, 32, 0.5),
+           (7424, 256, 512, 32, 0.5), (8192, 256, 512, 16, 0.8)]
+
+
 @pytest.mark.parametrize("shape", SHAPES)
 @pytest.mark.parametrize("dtype", [m.DType.F16, m.DType.BF16])
 @pytest.mark.parametrize("hint", ["right", "unknown", "none", "many"])
