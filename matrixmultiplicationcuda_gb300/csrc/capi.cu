@@ -293,7 +293,8 @@ namespace spmm {
 //     mma.sync where there is next to nothing to do (1024^2, 8 %: 3.8 against
 //     5.6).
 //   32- and 16-row blocks: mma.sync, whose CTAs are small, unless rows are known
-//     to be long, where a tcgen05 CTA's deeper ring pays: 32 rows, 8192^2, 8 %
+//     to be long, where a tcgen05 CTA's deeper ring pays (mma.sync taking single
+//     blocks; groups of four gain it up to 10 % on even rows): 32 rows, 8192^2, 8 %
 //     (41 blocks a row), N 512: 18.2 against 28.8; 1 % (5 a row): 8.8 against
 //     8.5. 16 rows, 8 %: 26.5 against 30.4; 1 %: 11.5 against 9.2; 8192^2 with
 //     log-normal rows, 8 %: 51 against 123. Its column tile is 256 wide, so
@@ -313,11 +314,11 @@ namespace spmm {
 //   e4m3: mma.sync or, where converts_e4m3 says so, the tcgen05 pipeline with
 //     e4m3 converted to fp16; both take any block scale (the block-scaled MMA,
 //     which a caller may ask for, is faster but needs powers of two). 16 rows and
-//     2048 items or more: mma.sync's 256-column tile (8192^2, 10 %, N 1024: 95
-//     against 119 for 128 columns; 2 % and log-normal rows, N 2048: 58 against 71;
-//     16384 x 4096, 2 %, N 512: 14.8 against 17.5). With fewer, 128 columns
-//     spread long rows further (16384 x 4096, log-normal, N 256: 20.6 against
-//     24.2), as where half of the last 256 would be empty (N 272: 14.1, 14.4).
+//     2048 items or more: mma.sync's 256-column tile (8192^2, 10 %, N 1024: 80
+//     against 102 for 128 columns; 2 % and log-normal rows, N 2048: 48 against 59;
+//     16384 x 4096, 2 %, N 512: 14.0 against 16.2). With fewer, 128 columns
+//     spread long rows further (16384 x 4096, log-normal, N 256: 16.4 against
+//     19.0), as where half of the last 256 would be empty (N 272: 13.2, 14.2).
 spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnzb) {
   spmm_config c;
   std::memset(&c, 0, sizeof(c));
@@ -366,16 +367,16 @@ spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnz
 
 // Whether an e4m3 product of known size runs converted to fp16 in the tcgen05
 // pipeline instead of on mma.sync (us, converted against mma.sync):
-//   64 rows: 16384^2, 2 % (20 blocks a row), N 512: 25.3, 34.3; 8192^2, 10 %, N
-//     1024: 47.6, 73.4; 32 rows: 60.9, 87.9; 8192^2 with log-normal rows, 3 %, N
-//     1024: 64 rows 32.4, 43.2, 32 rows 31.0, 44.4.
-//   Short rows do not fill its ring: 64 rows, 8192^2, 2 % (10 a row): 17.7, 19.9
-//     at N 1024, but 1 % (5 a row), N 512: 10.0, 9.2; 32 rows: 10.6, 9.5.
+//   64 rows: 16384^2, 2 % (20 blocks a row), N 512: 25.2, 32.4; 8192^2, 10 %, N
+//     1024: 47.4, 69.7; 32 rows: 61.0, 79.5; 8192^2 with log-normal rows, 3 %, N
+//     1024: 64 rows 32.0, 40.0, 32 rows 30.5, 41.4.
+//   Short rows do not fill its ring: 64 rows, 8192^2, 2 % (10 a row): 17.3, 19.7
+//     at N 1024, but 1 % (5 a row), N 512: 10.0, 9.0; 32 rows: 10.6, 8.9.
 //   With fewer items than CTAs run at once the longest rows bound both, and
 //     mma.sync's narrower tiles spread them further: 64 rows, 8192^2 with
-//     log-normal rows, N 512 (256 items): 45.6, 44.6.
-//   Its tile is 256 wide: 32 rows, 16384 x 8192, 5 %, N 272: 39.8, 35.8.
-//   16 rows: slower (8192^2, 10 %, N 1024: 108, 95 with mma.sync's 256-column tile).
+//     log-normal rows, N 512 (256 items): 45.6, 42.0.
+//   Its tile is 256 wide: 32 rows, 16384 x 8192, 5 %, N 272: 39.8, 34.8.
+//   16 rows: slower (8192^2, 10 %, N 1024: 108, 80 with mma.sync's 256-column tile).
 bool converts_e4m3(int bR, int M, int N, long long nnzb) {
   if (bR == 16 || nnzb < 0 || N <= 128 || (N > 256 && N <= 384)) return false;
   const long long items = (long long)(M / bR) * ((N + 255) / 256);
