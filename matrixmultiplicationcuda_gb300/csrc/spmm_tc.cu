@@ -41,6 +41,7 @@
 #include "csr.cuh"
 #include "internal.h"
 #include "ptx.cuh"
+#include "ring_rules.h"
 #include "spmm_mma.cuh"
 #include "tcgen05.cuh"
 
@@ -215,8 +216,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
   using Cfg = TcCfg<BR, NT, STAGES, MODE, ACC, G, FEED>;
   constexpr int kASource = FEED == kFeedConvert ? BR * 16 : Cfg::kABytes;   // bytes of a block in A's values
   constexpr bool GATHER = FEED == kFeedGather, CONVERT = FEED == kFeedConvert;
-  constexpr int kQ = 4;                       // item hand-off ring depth
-  constexpr int kBIssuers = 4;
+  constexpr int kQ = kItemRing;               // item hand-off ring depth
   constexpr int kScaleWriter = 3;             // e4m3: the B issuer that writes the scale tiles
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       // the lead's arrive (it expects the whole group's bytes); e4m3 also B
       // issuer 0's, after it has written the group's scale tiles
       // (with gather blocks: every lane of every B issuer, in every group)
-      // (converted e4m3: each B issuer, in every group)
-      mbar_init(full0 + 8 * s, Cfg::kE4 ? 2 : GATHER ? 1 + 32 * kBIssuers : CONVERT ? kBIssuers : 1);
+      // (converted e4m3: each B issuer and the lead, in every group)
+      mbar_init(full0 + 8 * s, Cfg::kE4 ? 2 : GATHER ? 1 + 32 * kBIssuers : CONVERT ? kConvertFullArrivals : 1);
       mbar_init(empty0 + 8 * s, Cfg::kIssuers);   // each MMA issuer's commit
     }
     for (int b = 0; b < 2; ++b) {
@@ -478,9 +478,13 @@ __global__ void __launch_bounds__(kTcThreads, 2)
               failed = true;
               break;
             }
-            // (the B issuers convert A's blocks too; the wait above keeps the claims' pace)
-            if constexpr (CONVERT) continue;
             const uint32_t fb = full0 + 8 * s;
+            if constexpr (CONVERT) {
+              // The B issuers convert A's blocks too. The wait above keeps the
+              // claims' pace; the arrival keeps the group from being consumed before it.
+              mbar_arrive(fb);
+              continue;
+            }
             // (with gather blocks the B issuers expect their panels' bytes themselves)
             mbar_arrive_expect_tx(fb, (uint32_t)(n * (Cfg::kABytes + (GATHER ? 0 : Cfg::kPanelBytes)) * Cfg::kParts));
             uint8_t* a_dst = smem + (size_t)s * Cfg::kStage;
