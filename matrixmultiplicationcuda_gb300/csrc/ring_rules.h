@@ -2,6 +2,13 @@
 // from the kernel so that a model of the protocol on the CPU runs the kernel's own
 // (tests/test_convert_ring.py).
 #pragma once
+#include <cstdint>
+
+#ifdef __CUDACC__
+#define SPMM_RULE __host__ __device__ constexpr
+#else
+#define SPMM_RULE constexpr
+#endif
 
 namespace spmm {
 
@@ -16,4 +23,14 @@ constexpr int kBIssuers = 4;    // B-issuing warps
 // items never comes.
 constexpr int kConvertFullArrivals = kBIssuers + 1;
 
+// Converted e4m3: a B issuer copies groups ahead of those it converts, across
+// items. Whether it may wait for an entry of the item ring that lies `ahead`
+// entries after the one whose group it has to convert next. The lead publishes
+// entry e once entry e - kItemRing has been read, and the MMA threads and the
+// epilogue read that one after finishing entry e - kItemRing - 1; an issuer that
+// waits for e with a group of that entry or an older one unconverted waits for
+// itself (items without blocks bring it there: they hold no group).
+SPMM_RULE bool may_wait_for_entry(uint32_t ahead) { return ahead <= (uint32_t)kItemRing; }
+
 }  // namespace spmm
+#undef SPMM_RULE

@@ -572,6 +572,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       constexpr int kDepth = Cfg::kDepth, kPer = kBIssuers / G, kRows = 16 / kPer, kARows = BR / kPer;
       constexpr int kCopies = Cfg::kCopies;
       static_assert(!CONVERT || (NT == 256 && kARows <= 32 && kBIssuers % G == 0), "the lane maps below");
+      static_assert(!CONVERT || (kDepth >= 2 && kDepth <= 3), "the waits for a group's copies below");
       const int myb = bidx / kPer, part = bidx % kPer;
       // Lane: 16 columns (a 16-byte chunk c) of rows r0, r0 + 2, ...: eight lanes
       // hold four chunks of two rows, whose fp16 stores fall on all banks.
@@ -583,12 +584,16 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       const uint32_t b_off = Cfg::kAStage + (c >> 2) * Cfg::kBoxBytes + r0 * 128;
       const uint32_t raw0 = smem_u32(smem) + STAGES * Cfg::kStage + bidx * (kDepth * Cfg::kRawGroup);
       // the copying end of the stream
-      uint32_t it = 0, copied = 0, has = 0;   // groups copied; bit g % 32: group g holds a block of this issuer
+      uint32_t it = 0, copied = 0, gs = 0;    // next entry of the item ring; groups copied, converted
+      uint32_t has = 0, entries = 0;          // bit g % 32: group g holds a block of this issuer; byte g % 4: its entry
       int j0 = 0, end = 0, base = 0, cols = 0, next_cols = 0;   // next group; lane's column indices from base, base + 32
       const uint8_t* bcol = bsrc;
       bool done = false;
-      auto copy_group = [&]() {
+      // One more group, if there is one (its copies are one cp.async group). False
+      // at the end of the items, and where the next item may not be waited for yet.
+      auto copy_group = [&]() -> bool {
         while (!done && j0 >= end) {
+          if (copied != gs && !may_wait_for_entry((it - (entries >> (8 * (gs & 3)))) & 255u)) return false;
           int item = -1, start = 0, e = 0, nt = 0, ok = 1;
           if (lane == 0) ok = read_item(it, &item, &start, &e, 4u, &nt) ? 1 : 0;
           ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -603,41 +608,45 @@ __global__ void __launch_bounds__(kTcThreads, 2)
           cols = base + lane < end && !done ? __ldg(p.col_idx + base + lane) : 0;
           next_cols = base + 32 + lane < end && !done ? __ldg(p.col_idx + base + 32 + lane) : 0;
         }
-        if (!done) {
-          if (j0 - base == 32) {
-            base = j0;
-            cols = next_cols;
-            next_cols = base + 32 + lane < end ? __ldg(p.col_idx + base + 32 + lane) : 0;
-          }
-          const int j = j0 + myb;
-          has &= ~(1u << (copied & 31));
-          if (j < end) {
-            has |= 1u << (copied & 31);
-            const int col = __shfl_sync(0xffffffffu, cols, j - base);
-            const uint32_t raw = raw0 + (copied % kDepth) * Cfg::kRawGroup + lane * 16;
-            if (lane < kARows) cp_async16(raw, asrc + (long long)j * (BR * 16));
-            if ((unsigned)col < (unsigned)(p.K >> 4)) {
-              const uint8_t* src = bcol + (long long)col * 16 * p.ldb;
-#pragma unroll
-              for (int k = 0; k < kCopies; ++k) cp_async16(raw + 512 * (k + 1), src + 2 * k * p.ldb);
-            } else {   // not a block column of A: rows of zeros, as a TMA copy reads them
-#pragma unroll
-              for (int k = 0; k < kCopies; ++k) st_shared_v4(raw + 512 * (k + 1), make_uint4(0u, 0u, 0u, 0u));
-            }
-            if (lane == 0) cp_async4(raw + 512 * (kCopies + 1), p.scales + j);
-          }
-          ++copied;
-          j0 += G;
+        if (done) return false;
+        if (j0 - base == 32) {
+          base = j0;
+          cols = next_cols;
+          next_cols = base + 32 + lane < end ? __ldg(p.col_idx + base + 32 + lane) : 0;
         }
+        const int j = j0 + myb;
+        has &= ~(1u << (copied & 31));
+        const uint32_t sh = 8 * (copied & 3);
+        entries = (entries & ~(255u << sh)) | (((it - 1) & 255u) << sh);
+        if (j < end) {
+          has |= 1u << (copied & 31);
+          const int col = __shfl_sync(0xffffffffu, cols, j - base);
+          const uint32_t raw = raw0 + (copied % kDepth) * Cfg::kRawGroup + lane * 16;
+          if (lane < kARows) cp_async16(raw, asrc + (long long)j * (BR * 16));
+          if ((unsigned)col < (unsigned)(p.K >> 4)) {
+            const uint8_t* src = bcol + (long long)col * 16 * p.ldb;
+#pragma unroll
+            for (int k = 0; k < kCopies; ++k) cp_async16(raw + 512 * (k + 1), src + 2 * k * p.ldb);
+          } else {   // not a block column of A: rows of zeros, as a TMA copy reads them
+#pragma unroll
+            for (int k = 0; k < kCopies; ++k) st_shared_v4(raw + 512 * (k + 1), make_uint4(0u, 0u, 0u, 0u));
+          }
+          if (lane == 0) cp_async4(raw + 512 * (kCopies + 1), p.scales + j);
+        }
+        ++copied;
+        j0 += G;
         cp_async_commit();
+        return true;
       };
       auto half8 = [](uint32_t x, uint32_t y) {   // 8 e4m3 -> 8 fp16
         return make_uint4(e4m3x2_to_f16x2(x), e4m3x2_to_f16x2(x >> 16), e4m3x2_to_f16x2(y), e4m3x2_to_f16x2(y >> 16));
       };
 #pragma unroll 1
-      for (int d = 0; d < kDepth; ++d) copy_group();
+      for (;; ++gs) {
 #pragma unroll 1
-      for (uint32_t gs = 0; gs < copied; ++gs) {
+        while (copied - gs < (uint32_t)kDepth && copy_group()) {
+        }
+        if (copied == gs) break;   // (with nothing left to convert the next item is always waited for)
         const int s = (int)(gs % STAGES);
         int bad = 0;
         if (lane == 0 && gs >= (uint32_t)STAGES &&
@@ -646,7 +655,13 @@ __global__ void __launch_bounds__(kTcThreads, 2)
           bad = 1;
         }
         if (__shfl_sync(0xffffffffu, bad, 0)) break;
-        cp_async_wait_group<kDepth - 1>();
+        // group gs has landed: all but the groups copied after it
+        if (copied - gs == (uint32_t)kDepth)
+          cp_async_wait_group<kDepth - 1>();
+        else if (copied - gs == 2)
+          cp_async_wait_group<1>();
+        else
+          cp_async_wait_group<0>();
         __syncwarp();   // the slot is free for every lane; lane 0's copy of the scale has landed
         if ((has >> (gs & 31)) & 1) {
           const uint32_t slot = smem_u32(smem + (size_t)s * Cfg::kStage);
@@ -688,7 +703,6 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(full0 + 8 * s);
-        copy_group();
       }
       cp_async_wait_all();
     };

@@ -20,7 +20,8 @@ def rules(tmp_path_factory):
     src = d / "rules.cpp"
     src.write_text('#include "ring_rules.h"\nextern "C" {\nint entries() { return spmm::kItemRing; }\n'
                    'int issuers() { return spmm::kBIssuers; }\n'
-                   'int arrivals() { return spmm::kConvertFullArrivals; }\n}\n')
+                   'int arrivals() { return spmm::kConvertFullArrivals; }\n'
+                   'int may_wait(unsigned ahead) { return spmm::may_wait_for_entry(ahead); }\n}\n')
     so = d / "rules.so"
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, str(src), "-o", str(so)], check=True)
     return ctypes.CDLL(str(so))
@@ -49,8 +50,9 @@ class Cta:
     """items: groups of each item of one CTA, in order. A role yields the barrier
     and parity that it waits for."""
 
-    def __init__(self, rules, items, stages, arrivals=None):
+    def __init__(self, rules, items, stages, arrivals=None, may_wait=None):
         self.items, self.stages = items, stages
+        self.may_wait = may_wait or rules.may_wait
         self.Q, self.issuers = rules.entries(), rules.issuers()
         arrivals = rules.arrivals() if arrivals is None else arrivals
         self.lead_arrives = arrivals > self.issuers
@@ -99,17 +101,19 @@ class Cta:
                 gs += 1
 
     def issuer(self, me):
-        it, left, copied, done, gs = 0, 0, 0, False, 0
+        it = left = gs = 0
+        done, ahead = False, []   # entries of the groups copied and not yet converted
         while True:
-            while not done and copied - gs < self.stages:
-                while not done and left == 0:
+            while len(ahead) < self.stages:
+                while not done and left == 0 and (not ahead or self.may_wait(it - ahead[0])):
                     left = yield from self.read(it)
                     it += 1
                     done = left < 0
-                if not done:
-                    left -= 1
-                    copied += 1
-            if copied == gs:
+                if done or left == 0:
+                    break
+                left -= 1
+                ahead.append(it - 1)
+            if not ahead:
                 return
             s = gs % self.stages
             if gs >= self.stages:
@@ -118,6 +122,7 @@ class Cta:
             self.slot[s][me] = gs
             self.full[s].arrive()
             gs += 1
+            ahead.pop(0)
 
     def mma(self, me):
         gs = it = 0
@@ -180,3 +185,24 @@ def test_items_with_blocks(rules, items, stages):
 def test_a_lead_that_waits_without_arriving_is_left_behind(rules, stages):
     with pytest.raises(Deadlock):
         run_all(rules, [20, 1], stages, arrivals=rules.issuers())
+
+
+# items without blocks: after a long row, at the end, between rows of one group, everywhere
+@pytest.mark.parametrize("stages", [2, 3])
+@pytest.mark.parametrize("items", [[5, 0, 0, 0, 0], [1] + [0] * 16 + [1], [0] * 9, [20] + [0] * 5 + [3] + [0] * 4 + [1, 2],
+                                   [3, 0, 1, 0, 0, 1, 0, 0, 4], [1, 0, 1, 0, 0, 1, 0, 0, 0, 1, 0, 0, 0, 0, 1]])
+def test_items_without_blocks(rules, items, stages):
+    run_all(rules, items, stages)
+
+
+def test_random_items(rules):
+    for seed in range(400):
+        rng = random.Random(seed)
+        items = [rng.choice((0, 0, 0, 1, 1, 2, 3, 5)) for _ in range(rng.randrange(1, 24))]
+        Cta(rules, items, rng.choice((2, 3))).run(rng, rng.randrange(-1, 11))
+
+
+@pytest.mark.parametrize("stages,items", [(2, [1, 0, 0, 0, 0]), (3, [1, 0, 0, 0, 0]), (3, [3, 0, 1, 0, 0, 1, 0, 0, 4])])
+def test_an_issuer_that_always_waits_for_the_next_item_waits_for_itself(rules, stages, items):
+    with pytest.raises(Deadlock):
+        run_all(rules, items, stages, may_wait=lambda ahead: True)

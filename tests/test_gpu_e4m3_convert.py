@@ -85,3 +85,45 @@ def test_sixteen_rows_many_items(dev, N):
     terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
     bound = terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs())
     assert ((C.double() - Ad @ Bd).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("bR", [32, 64])
+@pytest.mark.parametrize("N,shape", [(512, "tail"), (1280, "holes"), (256, "runs"), (4096, "ones")])
+def test_converted_product_with_many_empty_rows(dev, bR, N, shape):
+    """More items without blocks in a row than the item ring has entries: after
+    long rows, at the end of the grid, between rows of one block; bound as above."""
+    tiles = -(-N // 256)
+    MB, KB = max(48, -(-1400 // tiles)), 96
+    rng = np.random.default_rng(N + bR)
+    keep = rng.uniform(size=(MB, KB)) < 0.7
+    if shape == "tail":
+        keep[MB // 3:] = False
+    elif shape == "holes":
+        keep[rng.uniform(size=MB) < 0.5] = False
+    elif shape == "runs":                   # five empty rows at the start, then eight at a time
+        keep[np.arange(MB) % 16 > 6] = False
+        keep[np.arange(MB) % 16 == 15] = True
+        keep[1:6] = False
+    else:                                   # rows of one block among empty ones
+        keep[rng.uniform(size=MB) < 0.4] = False
+        keep[rng.uniform(size=MB) < 0.3, 1:] = False
+    assert keep.sum() >= 10 * MB and MB * tiles >= 304
+    g = torch.Generator(device=dev).manual_seed(N)
+    n = int(keep.sum())
+    vals = torch.randint(0, 0x7f, (n, bR, 16), generator=g, device=dev, dtype=torch.uint8)
+    sc = torch.exp2(torch.randint(-9, 1, (n,), generator=g, device=dev).float())
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a.astype(np.int32))).to(dev)
+    A = m.BCSR(MB * bR, KB * 16, bR, 16, t(np.concatenate([[0], np.cumsum(keep.sum(1))])), t(np.nonzero(keep)[1]),
+               vals.view(-1), m.DType.E4M3, None, sc)
+    B = torch.randint(0, 0x7f, (KB * 16, N), generator=g, device=dev, dtype=torch.uint8)
+    Ad = torch.zeros(MB, KB, bR, 16, dtype=torch.float64, device=dev)
+    Ad[torch.from_numpy(keep).to(dev)] = (vals.view(torch.float8_e4m3fn).float() * sc[:, None, None]).half().double()
+    Ad = Ad.permute(0, 2, 1, 3).reshape(MB * bR, KB * 16)
+    Bd = B.view(torch.float8_e4m3fn).double()
+    terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
+    ref, bound = Ad @ Bd, terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs())
+    for _ in range(3):
+        C = torch.full((MB * bR, N), float("nan"), device=dev)
+        m.spmm(A, B, C=C)
+        m.device_error_check()
+        assert ((C.double() - ref).abs() <= bound).all()
