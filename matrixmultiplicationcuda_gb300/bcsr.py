@@ -298,8 +298,20 @@ def dense_to_bcsr(A_half, bR=16, bC=16, stream=None):
     rp = torch.empty(MB + 1, dtype=torch.int32, device=A_half.device)
     masks = torch.empty(max(lib().spmm_dense_to_bcsr_mask_words(M, K, bR, bC), 0), dtype=torch.int32,
                         device=A_half.device)
-    if stream is not None:
-        masks.record_stream(stream)   # its last reader runs there
+    side = None   # another stream than the one whose memory pool the tensors come from
+    current = torch.cuda.current_stream(A_half.device) if stream is not None else None
+    if stream is not None and stream.cuda_stream != current.cuda_stream:
+        side = stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(stream.cuda_stream)
+
+    def use(*tensors):
+        # their memory may still be in use by what is queued on the current
+        # stream, and may be given away there before `side` is done with it
+        if side is not None:
+            side.wait_stream(current)
+            for t in tensors:
+                t.record_stream(side)
+
+    use(rp, masks)
     nnzb = ctypes.c_longlong(0)
     s = stream_handle(stream)
     check(lib().spmm_dense_to_bcsr_count_masks(_ptr(A_half), M, K, lda, bR, bC, _ptr(rp), _ptr(masks),
@@ -307,6 +319,7 @@ def dense_to_bcsr(A_half, bR=16, bC=16, stream=None):
     ci = torch.empty(max(nnzb.value, 0), dtype=torch.int32, device=A_half.device)
     vals = torch.empty(max(nnzb.value, 0) * bR * bC, dtype=torch.float16, device=A_half.device)
     if nnzb.value:
+        use(ci, vals)
         check(lib().spmm_dense_to_bcsr_fill_masks(_ptr(A_half), M, K, lda, bR, bC, _ptr(rp), _ptr(masks), _ptr(ci),
                                                   _ptr(vals), s))
     return rp, ci, vals
