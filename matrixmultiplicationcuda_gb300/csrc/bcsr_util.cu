@@ -5,6 +5,7 @@
 #include <cuda_fp8.h>
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include "internal.h"
 #include "ptx.cuh"
 
@@ -451,20 +452,52 @@ static spmm_status conv_checks(const void* A, int M, int K, int lda, int bR, int
   return SPMM_OK;
 }
 
-// The calling thread's word of pinned memory that a scan writes its total to:
-// a copy into pageable memory would go through a staging buffer of the driver.
-static int* host_total() {
-  struct Word {
-    int* p = nullptr;
-    ~Word() {
-      if (p) cudaFreeHost(p);
+// A word of pinned memory that a call's scan writes its total to (a copy into
+// pageable memory would go through a staging buffer of the driver). The words
+// are one 4 KB block that stays for the process: nothing is allocated or freed as
+// threads come and go, which would break a graph capture of another thread. NULL
+// when all 64 are in use or there is no pinned memory; the caller then copies.
+class PinnedWord {
+ public:
+  PinnedWord() {
+    std::lock_guard<std::mutex> lk(mutex());
+    if (!block() && !tried()) {
+      tried() = true;
+      // (this thread's allocation must not end a capture of another one)
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      void* p = nullptr;
+      if (cudaHostAlloc(&p, kWords * kStride * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
+        block() = static_cast<int*>(p);
+      else
+        cudaGetLastError();
+      cudaThreadExchangeStreamCaptureMode(&mode);
     }
-  };
-  static thread_local Word w;
-  if (!w.p && cudaHostAlloc(reinterpret_cast<void**>(&w.p), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
-    w.p = nullptr;
-  return w.p;
-}
+    for (int w = 0; block() && w < kWords && slot_ < 0; ++w)
+      if (!(used() >> w & 1u)) {
+        used() |= 1ull << w;
+        slot_ = w;
+      }
+  }
+  ~PinnedWord() {
+    if (slot_ < 0 || keep_) return;
+    std::lock_guard<std::mutex> lk(mutex());
+    used() &= ~(1ull << slot_);
+  }
+  PinnedWord(const PinnedWord&) = delete;
+  PinnedWord& operator=(const PinnedWord&) = delete;
+  int* get() const { return slot_ < 0 ? nullptr : block() + slot_ * kStride; }
+  void keep() { keep_ = true; }   // a kernel may still write it: not given to another call
+
+ private:
+  static constexpr int kWords = 64, kStride = 16;   // a cache line each
+  static std::mutex& mutex() { static std::mutex m; return m; }
+  static int*& block() { static int* p = nullptr; return p; }
+  static unsigned long long& used() { static unsigned long long u = 0; return u; }
+  static bool& tried() { static bool t = false; return t; }
+  int slot_ = -1;
+  bool keep_ = false;
+};
 
 static int mask_groups(int K, int bC) {
   const int KB = K / bC, gblk = 32 / (bC / 8);
@@ -475,8 +508,7 @@ static int mask_groups(int K, int bC) {
 static spmm_status count_blocks(const void* A, int M, int K, int lda, int bR, int bC, uint32_t* masks, int* row_ptr,
                                 long long* nnzb_out, cudaStream_t s) {
   const int MB = M / bR, KB = K / bC, ngroups = mask_groups(K, bC);
-  int* total = host_total();
-  if (!total) return fail(SPMM_ERR_CUDA, "no pinned memory for the block count");
+  PinnedWord total;
   // counts go to row_ptr[1..MB] first and the scan rewrites row_ptr in place:
   // each thread reads a count before it writes that slot, and the threads'
   // slots are disjoint
@@ -491,9 +523,16 @@ static spmm_status count_blocks(const void* A, int M, int K, int lda, int bR, in
     SPMM_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * MB, s));
   }
   SPMM_CUDA_TRY(launch_kernel(&k_scan_counts, dim3(1), dim3(1024), 0, s, static_cast<const int*>(counts), row_ptr, MB,
-                              static_cast<const uint32_t*>(KB > 0 ? masks : nullptr), ngroups, total));
-  SPMM_CUDA_TRY(cudaStreamSynchronize(s));
-  *nnzb_out = *static_cast<volatile int*>(total);
+                              static_cast<const uint32_t*>(KB > 0 ? masks : nullptr), ngroups, total.get()));
+  int copied = 0;
+  if (!total.get())
+    SPMM_CUDA_TRY(cudaMemcpyAsync(&copied, row_ptr + MB, sizeof(int), cudaMemcpyDeviceToHost, s));
+  const cudaError_t ce = cudaStreamSynchronize(s);
+  if (ce != cudaSuccess) {
+    total.keep();
+    return cuda_fail(ce, "cudaStreamSynchronize(s)");
+  }
+  *nnzb_out = total.get() ? *static_cast<volatile int*>(total.get()) : copied;
   return SPMM_OK;
 }
 
