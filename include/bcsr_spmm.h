@@ -49,7 +49,7 @@ typedef struct spmm_config {
                     3 = tcgen05 pipeline for 64-row blocks with M = 64 UMMAs       */
   int n_tile;    /* output columns per CTA tile: 64, 128 or 256 (0 = auto)           */
   int stages;    /* pipeline depth 2..8 (0 = auto)                                   */
-  int ctas_per_sm; /* persistent grid = SMs x this (0 = auto)                          */
+  int ctas_per_sm; /* CTAs that run per SM (0 = as many as fit)                         */
   int acc_buffers; /* tcgen05: TMEM accumulators per CTA, 1 or 2 (0 = auto)          */
   int schedule;    /* tcgen05: 0 = static item stride, 1 = dynamic (a CTA takes
                       over blocks of its grid that have not started),

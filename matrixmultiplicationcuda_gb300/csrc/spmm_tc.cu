@@ -1359,7 +1359,6 @@ spmm_status launch_tc(const LaunchRequest& r) {
   if (p.n_items == 0) return SPMM_OK;
   if (p.split > 1)
     SPMM_CUDA_TRY(cudaMemset2DAsync(r.C, (size_t)r.ldc * 4, 0, (size_t)r.N * 4, A.M, r.stream));
-  SPMM_CUDA_TRY(ensure_smem_attr(reinterpret_cast<const void*>(e->fn), (int)e->smem));
   // CTAs per SM from the real limits: TMEM columns (512 per SM), shared memory
   // per SM, and the two CTAs the launch bounds budget registers for. (The
   // runtime's occupancy query reports one CTA per SM for this kernel, while two
@@ -1367,23 +1366,27 @@ spmm_status launch_tc(const LaunchRequest& r) {
   const int smem_sm = smem_per_sm();
   const int tmem_fit = 512 / e->tmem_cols;
   const int smem_fit = smem_sm / (int)(e->smem + 1024);
-  int per_sm = std::min(2, std::min(tmem_fit, smem_fit));
-  if (r.cfg.ctas_per_sm > 0 && r.cfg.ctas_per_sm < per_sm) per_sm = r.cfg.ctas_per_sm;
-  if (per_sm < 1) per_sm = 1;
+  const int fit = std::max(1, std::min(2, std::min(tmem_fit, smem_fit)));
+  const int per_sm = r.cfg.ctas_per_sm > 0 ? std::min(fit, r.cfg.ctas_per_sm) : fit;
   // later items: a plan's queue, or on request the grid's pending blocks (one
-  // block per item; a request for fewer CTAs per SM keeps the static stride,
-  // whose grid it sets)
+  // block per item)
   p.queue = r.items ? r.queue : nullptr;
-  p.dynamic = !r.items && r.cfg.schedule >= 1 && r.cfg.ctas_per_sm <= 0 ? 1 : 0;
+  p.dynamic = !r.items && r.cfg.schedule >= 1 ? 1 : 0;
+  // One block per item leaves the number of CTAs per SM to the hardware: where a
+  // caller wants one and two fit, half an SM's shared memory keeps the second out.
+  // (The kernel's limit is set once for both sizes: it is per kernel, not per launch.)
+  const size_t smem_one = std::max(e->smem, (size_t)smem_sm / 2);
+  SPMM_CUDA_TRY(ensure_smem_attr(reinterpret_cast<const void*>(e->fn), (int)smem_one));
+  const size_t smem = p.dynamic && per_sm < fit ? smem_one : e->smem;
   long long grid = (long long)sm_count() * per_sm;
   if (grid > p.n_items || p.dynamic) grid = p.n_items;
   if (std::getenv("SPMM_DEBUG"))
     std::fprintf(stderr,
                  "[spmm] tcgen05 bR=%d nt=%d stages=%d acc=%d group=%d smem=%zu tmem=%d per_sm=%d grid=%lld "
                  "items=%d panel3d=%d dynamic=%d queue=%d claim_ahead=%d inputs_ready=%d split=%d\n",
-                 A.bR, nt, e->stages, e->acc, e->group, e->smem, e->tmem_cols, per_sm, grid, p.n_items, panel3d,
+                 A.bR, nt, e->stages, e->acc, e->group, smem, e->tmem_cols, per_sm, grid, p.n_items, panel3d,
                  p.dynamic, p.queue != nullptr, p.claim_ahead, p.inputs_ready, p.split);
-  SPMM_CUDA_TRY(launch_kernel(e->fn, dim3((unsigned)grid), dim3(kTcThreads), e->smem, r.stream, tmA1, tmAg, tmAlo1,
+  SPMM_CUDA_TRY(launch_kernel(e->fn, dim3((unsigned)grid), dim3(kTcThreads), smem, r.stream, tmA1, tmAg, tmAlo1,
                               tmAlog, tmB, tmBlo, p));
   return SPMM_OK;
 }
