@@ -282,35 +282,49 @@ spmm_status spmm_device_error_check(void* stream) {
 namespace spmm {
 
 // What a product with no configuration runs, from its sizes and (nnzb >= 0) the
-// number of stored blocks. Times in us on one GB300, back to back, fp16, the
-// line's two sides:
-//   64-row blocks: tc512 (two accumulators) from 1024 columns and 256 tiles on
-//     (8192^2, 20 %, N 1024: 41.8 against 48.6 for the 64-row pipeline and 48.9
-//     for tc256; at half as many tiles 11.4 against 12.0, with log-normal rows
-//     35 against 31); else the 64-row pipeline (8192^2, 8 %, N 128: 9.7 against
-//     11.5 for tc128; log-normal, N 512: 47 against 62 for tc256), but tc256
-//     where rows are known to be short (1 %, N 512: 7.8 against 8.5) and
-//     mma.sync where there is next to nothing to do (1024^2, 8 %: 3.8 against
-//     5.6).
-//   32- and 16-row blocks: mma.sync, whose CTAs are small, unless rows are known
-//     to be long, where a tcgen05 CTA's deeper ring pays (mma.sync taking single
-//     blocks; groups of four gain it up to 10 % on even rows): 32 rows, 8192^2, 8 %
-//     (41 blocks a row), N 512: 18.2 against 28.8; 1 % (5 a row): 8.8 against
-//     8.5. 16 rows, 8 %: 26.5 against 30.4; 1 %: 11.5 against 9.2; 8192^2 with
-//     log-normal rows, 8 %: 51 against 123. Its column tile is 256 wide, so
-//     narrower products stay. With many items, so that its CTAs have a next one
-//     to overlap, it pays on shorter rows: 32 rows, 2 % (10 a row), N 1024: 17.0
-//     against 22.0, 5.7 a row 14.4, 16.6, log-normal, 1.2 %, N 512: 10.2, 12.8;
-//     16 rows, 10 a row, N 1024: 20.9, 22.0, log-normal, 15 a row, N 2048: 50, 63.
-//     On mma.sync, rows of six blocks and more take the ring of eight (a group
-//     of four in the time of two blocks, the 16-row tile of 256 columns only
-//     where its three CTAs per SM hold all items): 2048^2 log-normal, 16 rows, 6.6
-//     a row, N 512: 9.8 -> 7.2, 8192^2, N 104: 24.1 -> 18.7; the 256-column tile
-//     with more items: 8192^2, 6 a row, N 512: 9.7 against 10.2 with the larger
-//     ring. 64 columns or fewer then take the 128-column tile (4096^2, 12.7 a row:
-//     5.3 against 6.6) unless there are block rows enough (16384: 8.1, 7.9).
-//   split fp16, 64-row blocks above 128 columns: the 64-row pipeline (16384^2,
-//     2 %, N 512: 30.5 against 33.9 for tc256).
+// number of stored blocks. The lines stand where neither side of one was more
+// than 5 % slower than a single fixed kernel (the 128- or 256-column tcgen05
+// kernel for 64 rows, mma.sync with single blocks for 16 and 32), over 2000
+// products (M to 16384, K 256 to 16384, N 40 to 4096, 0.5 to 300 blocks a row;
+// even, random and log-normal rows; replayed ten at a time on one GB300). items:
+// block rows x 256-column tiles. Times in us, the line's two sides:
+//   64-row blocks, fp16 and bf16:
+//     - next to nothing to do (known): mma.sync. 43 rows of one block, N 104: 2.5
+//       (64-row pipeline 4.3, tc128 4.8). Not for long rows, whose blocks one CTA
+//       takes one by one: one row of 83, N 128: 19.0, tc128 12.4.
+//     - as many items as SMs at most: the 64-row pipeline, which gives an item a
+//       whole SM. 45 block rows, 97 blocks a row, N 512: 14.8, tc256 21.4; with
+//       more its last round is half empty: 237 rows of one block, N 512: 11.8,
+//       9.3; 184 rows of 61, N 120: 22.9, tc128 16.4.
+//     - 128 columns and fewer: tc128, and the 64-row pipeline (items as above)
+//       only for whole 64-column boxes: 83 rows of 39, N 40: 12.2, 10.1.
+//     - 512-column tiles from 1024 columns and 256 of them on: 206 rows of 47, N
+//       2048: 55 (64-row pipeline 66, tc256 68). Not for the shortest rows (known):
+//       230 of 0.7, N 1024: 16.3, tc256 15.3.
+//     - more than two items an SM and 8 or more blocks a row (known): the 64-row
+//       pipeline (144 rows of 30, N 776: 25.0, 26.5), else tc256 (254 rows of 1.4, N
+//       400: 11.8, 10.9). Rows of one or two blocks (known) take the static
+//       stride, as a claim costs more than they do: 10.2 against 10.9.
+//   split fp16 above 128 columns: the 64-row pipeline, but tc256 for more items
+//     than SMs with less than 6 blocks a row or an unknown number (57 rows of two,
+//     N 4096: 19.4, 14.0; but 190 rows of 19, N 512: 18.3, 22.8).
+//   32- and 16-row blocks: mma.sync, whose CTAs are small, with single blocks
+//     unless rows are known to be longer. From 5.5 blocks a row (8 with more items
+//     than SMs, 16 then with part boxes below 128 columns) a ring of eight in
+//     groups of four: one row of 12, N 64, 32 rows: 3.6, 4.4; 200 rows of 7, N 264:
+//     5.6, 5.2; 382 of 11.5, N 72: 8.4, 7.7. Its tile is 128 columns wide: up to
+//     64 columns only with few block rows (352 of 8, N 40: 7.9, 5.4; whole boxes
+//     to four per SM: 14.8 to 12.6 us at 626 rows of 40, 16 rows, but 11.0 from 10.5
+//     at 861 of 23). 16 rows: to two items an SM, the 256-column tile to three (206
+//     rows of 25, N 512: 8.3, 128 columns 11.4, single blocks 9.7).
+//     The longer the rows and the more the items, the better a tcgen05 CTA's
+//     deeper ring: 32 rows, few items: 40 a row (one of 83, N 128 stays; 50 rows of
+//     19, N 256: 6.8, 4.8 for the ring of eight), 20 with two an SM, 12 with more,
+//     5 with five (8192^2, 5.7 a row, N 1024: 14.4, 16.6). 16 rows: 64 (14 rows of
+//     17, N 512: 6.3, 4.1), not between two and three items an SM, where mma.sync's
+//     CTAs hold all (322 rows of 21, N 256: 10.5, 7.4), 12 from five (10 from seven)
+//     on: 8192^2, 10 a row, N 1024: 20.9, 22.0. Its tile is 256 columns wide, so
+//     the last one has to be at least half used.
 //   e4m3: mma.sync or, where converts_e4m3 says so, the tcgen05 pipeline with
 //     e4m3 converted to fp16; both take any block scale (the block-scaled MMA,
 //     which a caller may ask for, is faster but needs powers of two). 16 rows and
@@ -323,6 +337,9 @@ spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnz
   spmm_config c;
   std::memset(&c, 0, sizeof(c));
   const double row = nnzb >= 0 && M > 0 ? (double)nnzb * bR / M : -1.0;   // blocks per block row
+  const long long sms = sm_count();
+  // (rows not known: as with many)
+  const long long items = M > 0 ? (long long)(M / bR) * ((N + 255) / 256) : 1ll << 40;
   auto tc = [&](int kernel, int nt, int acc) {
     c.kernel = kernel;
     c.n_tile = nt;
@@ -330,37 +347,60 @@ spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnz
     c.schedule = 1;
     c.split_k = 1;
   };
-  if (dtype != SPMM_E4M3) {
-    if (bR == 64 && dtype == SPMM_F16_SPLIT) {
-      if (N <= 128)
-        tc(2, 128, 2);
+  auto tc256 = [&] {
+    tc(2, 256, 2);
+    if (row >= 0 && row < 2.5) c.schedule = 0;
+  };
+  const bool sixteen = dtype == SPMM_F16 || dtype == SPMM_BF16;
+  if (bR == 64 && dtype == SPMM_F16_SPLIT) {
+    if (N <= 128)
+      tc(2, 128, 2);
+    else if (items <= sms || row >= 6)
+      tc(3, 256, 0);
+    else
+      tc256();
+    return c;
+  }
+  if (bR == 64 && sixteen && !(nnzb >= 0 && nnzb <= 100 && row <= 8)) {
+    if (N <= 128) {
+      if (items <= sms && N % 64 == 0)
+        tc(3, 256, 0);
       else
-        tc(3, 256, 0);
-    } else if (bR == 64) {
-      const bool tiles512 = N >= 1024 && (N % 512 == 0 || N % 512 > 256) && (long long)(M / 64) * ((N + 511) / 512) >= 256;
-      if (tiles512)
-        tc(2, 512, 2);
-      else if (row >= 0 && nnzb > 100 && row < 8 && N > 128)
-        tc(2, 256, 2);
-      else if (nnzb < 0 || nnzb > 100)
-        tc(3, 256, 0);
-    } else if (dtype != SPMM_F16_SPLIT && N > 128) {
-      const long long items = (long long)(M / bR) * ((N + 255) / 256);
-      const bool whole = N <= 256 || N > 384;   // the last 256-column tile at least half used
-      if (row >= (bR == 16 ? 16 : 12) ||
-          (whole && (bR == 16 ? row >= 10 && items >= 1024 : row >= 5 && items >= 3ll * sm_count())))
-        tc(2, 256, 2);
+        tc(2, 128, 2);
+    } else if (!(row >= 0 && row < 2.5) && N >= 1024 && (N % 512 == 0 || N % 512 > 256) &&
+               (long long)(M / 64) * ((N + 511) / 512) >= 256) {
+      tc(2, 512, 2);
+    } else if (items <= sms || (items > 2 * sms && row >= 8)) {
+      tc(3, 256, 0);
+    } else {
+      tc256();
     }
-    if (c.kernel != 0) return c;
+    return c;
+  }
+  if (bR != 64 && sixteen && N > 128 && (N <= 256 || N > 384)) {   // the last 256-column tile at least half used
+    const double long_row = bR == 32 ? (items <= sms ? 40 : items <= 2 * sms ? 20 : items < 5 * sms ? 12 : 5)
+                                     : (items > 2 * sms && items <= 3 * sms ? 1e9 : items < 5 * sms ? 64 : items < 7 * sms ? 12 : 10);
+    if (row >= long_row) {
+      tc(2, 256, 2);
+      return c;
+    }
   }
   c.kernel = 1;
-  c.n_tile = bR == 64 && dtype != SPMM_E4M3 && dtype != SPMM_F16_SPLIT ? 64 : mma_default_nt(bR, dtype, N);
-  if (dtype == SPMM_E4M3 && bR == 16 && N > 128 && (N <= 256 || N > 384) && (long long)(M / 16) * ((N + 255) / 256) >= 2048)
-    c.n_tile = 256;
+  c.n_tile = bR == 64 && sixteen ? 64 : mma_default_nt(bR, dtype, N);
+  if (dtype == SPMM_E4M3 && bR == 16 && N > 128 && (N <= 256 || N > 384) && M > 0 && items >= 2048) c.n_tile = 256;
   c.stages = 4;
-  if (bR != 64 && (dtype == SPMM_F16 || dtype == SPMM_BF16) && row >= 5.5) {
-    if (c.n_tile == 64 && (N > 64 || M / bR < 4 * sm_count())) c.n_tile = 128;
-    if (c.n_tile == 128 || (c.n_tile == 256 && (M / 16) * ((N + 255ll) / 256) <= 3 * sm_count())) c.stages = 8;
+  if (bR != 64 && sixteen && row >= (items <= sms ? 5.5 : N < 128 && N % 64 ? 16 : 8)) {
+    if (N <= 128) {
+      if (c.n_tile != 64 || N > 64 || M / bR < (N % 64 == 0 ? 4 * sms : sms)) {
+        c.n_tile = 128;
+        c.stages = 8;
+      }
+    } else if (bR == 32 || items <= 2 * sms) {
+      c.n_tile = 128;
+      c.stages = 8;
+    } else if (items <= 3 * sms && c.n_tile == 256) {
+      c.stages = 8;
+    }
   }
   return c;
 }

@@ -85,3 +85,27 @@ def test_captured_and_replayed_by_two_streams(dev, shape):
     m.device_error_check()
     for C in Cs:
         assert ((C.double() - ref).abs() <= bound).all()
+
+
+# both sides of the lines for 64-row blocks: few blocks, as many items as SMs, whole
+# boxes, long rows in many items; split fp16 likewise
+LINES = [(576, 640, 104, 64, 0.2), (9664, 256, 128, 64, 0.5), (9664, 256, 136, 64, 0.1), (9792, 128, 64, 64, 0.6),
+         (19584, 128, 256, 64, 0.9), (19584, 512, 256, 64, 0.4), (19584, 256, 264, 64, 0.1)]
+
+
+@pytest.mark.parametrize("shape", LINES)
+@pytest.mark.parametrize("dtype", [m.DType.F16, m.DType.F16_SPLIT])
+@pytest.mark.parametrize("hint", ["right", "unknown"])
+def test_default_kernel_of_64_rows(dev, shape, dtype, hint):
+    M, K, N, bR, density = shape
+    A, B, ref, bound = problem(dev, M, K, N, bR, density, m.DType.F16, seed=M + N)
+    lo = None
+    if dtype == m.DType.F16_SPLIT:   # (low halves of zero: the product is the fp16 one)
+        A.dtype, A.vals_lo, lo = dtype, torch.zeros_like(A.vals), torch.zeros_like(B)
+    C = torch.full((M, N), float("nan"), device=dev)
+    a = A.desc()
+    b = m._lib.DenseDesc(B.data_ptr(), None if lo is None else lo.data_ptr(), 1.0, N)
+    n = A.nnzb if hint == "right" else -1
+    m.check(m.lib().spmm_bcsr_mm_nnzb(ctypes.byref(a), n, ctypes.byref(b), N, C.data_ptr(), N, None, m.stream_handle()))
+    m.device_error_check()
+    assert ((C.double() - ref).abs() <= bound).all()
