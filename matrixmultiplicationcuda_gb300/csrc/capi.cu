@@ -410,17 +410,24 @@ spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnz
 //   64 rows: 16384^2, 2 % (20 blocks a row), N 512: 25.2, 32.4; 8192^2, 10 %, N
 //     1024: 47.4, 69.7; 32 rows: 61.0, 79.5; 8192^2 with log-normal rows, 3 %, N
 //     1024: 64 rows 32.0, 40.0, 32 rows 30.5, 41.4.
-//   Short rows do not fill its ring: 64 rows, 8192^2, 2 % (10 a row): 17.3, 19.7
-//     at N 1024, but 1 % (5 a row), N 512: 10.0, 9.0; 32 rows: 10.6, 8.9.
+//   Short rows do not fill its ring, and with few items its last round of CTAs (two
+//     an SM) is short of work: 64 rows, 8192^2, 10 a row, N 1024 (512 items): 17.3,
+//     19.7, but 93 rows of 10, N 1024 (372): 15.1, 12.5; 32 rows: 166 rows of 11, N
+//     1008 (664): 16.7, 13.6, 164 of 52, N 400 (328): 34.5, 30.6, but 314 of 21, N
+//     512 (628): 21.3, 22.9, and 212 of 69, N 512 (424): 39, 48.
 //   With fewer items than CTAs run at once the longest rows bound both, and
 //     mma.sync's narrower tiles spread them further: 64 rows, 8192^2 with
 //     log-normal rows, N 512 (256 items): 45.6, 42.0.
-//   Its tile is 256 wide: 32 rows, 16384 x 8192, 5 %, N 272: 39.8, 34.8.
+//   Its tile is 256 wide: 32 rows, 16384 x 8192, 5 %, N 272: 39.8, 34.8; 94 rows of
+//     17, N 784: 17.1, 12.0; long rows: 422 of 55, N 784: 110, 112.
 //   16 rows: slower (8192^2, 10 %, N 1024: 108, 80 with mma.sync's 256-column tile).
 bool converts_e4m3(int bR, int M, int N, long long nnzb) {
   if (bR == 16 || nnzb < 0 || N <= 128 || (N > 256 && N <= 384)) return false;
-  const long long items = (long long)(M / bR) * ((N + 255) / 256);
-  return nnzb * bR >= 10ll * M && items >= 2ll * sm_count();
+  const long long items = (long long)(M / bR) * ((N + 255) / 256), sms = sm_count();
+  const double row = (double)nnzb * bR / M;
+  const bool whole = N % 256 == 0 || N % 256 > 128;   // the last tile at least half used
+  if (!whole && row < 40) return false;
+  return items >= 2.5 * sms && (row >= 24 || (items >= 3 * sms && row >= (bR == 64 ? 10 : 16)));
 }
 
 }  // namespace spmm

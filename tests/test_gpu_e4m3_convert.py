@@ -127,3 +127,34 @@ def test_converted_product_with_many_empty_rows(dev, bR, N, shape):
         m.spmm(A, B, C=C)
         m.device_error_check()
         assert ((C.double() - ref).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("bR,items,K,N,pad", [(32, 460, 400, 400, 16), (64, 460, 208, 768, 0), (32, 384, 640, 512, 0),
+                                              (64, 384, 640, 400, 32), (32, 384, 880, 784, 0), (64, 384, 880, 656, 0)])
+def test_converted_product_at_the_rule(dev, bR, items, K, N, pad):
+    """Sizes just inside spmm_bcsr_mm_nnzb's rule for the conversion (rows of at
+    least 10, 16, 24 and 40 blocks), part tiles of columns; bound as above."""
+    MB, KB = -(-items // -(-N // 256)), K // 16
+    rng = np.random.default_rng(N + K)
+    keep = rng.uniform(size=(MB, KB)) < 0.9
+    keep[2] = False
+    g = torch.Generator(device=dev).manual_seed(N + bR)
+    n = int(keep.sum())
+    vals = torch.randint(0, 0x7f, (n, bR, 16), generator=g, device=dev, dtype=torch.uint8)
+    vals ^= torch.randint(0, 2, (n, bR, 16), generator=g, device=dev, dtype=torch.uint8) << 7
+    sc = torch.rand(n, generator=g, device=dev) * 0.02 + 1e-4
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a.astype(np.int32))).to(dev)
+    A = m.BCSR(MB * bR, K, bR, 16, t(np.concatenate([[0], np.cumsum(keep.sum(1))])), t(np.nonzero(keep)[1]),
+               vals.view(-1), m.DType.E4M3, None, sc)
+    Bw = torch.full((K, N + pad), 0x7f, dtype=torch.uint8, device=dev)
+    Bw[:, :N] = torch.randint(0, 0x7f, (K, N), generator=g, device=dev, dtype=torch.uint8)
+    C = torch.full((MB * bR, N), float("nan"), device=dev)
+    m.spmm(A, Bw[:, :N], N=N, C=C)
+    m.device_error_check()
+    Ad = torch.zeros(MB, KB, bR, 16, dtype=torch.float64, device=dev)
+    Ad[torch.from_numpy(keep).to(dev)] = (vals.view(torch.float8_e4m3fn).float() * sc[:, None, None]).half().double()
+    Ad = Ad.permute(0, 2, 1, 3).reshape(MB * bR, K)
+    Bd = Bw[:, :N].contiguous().view(torch.float8_e4m3fn).double()
+    terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
+    bound = terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs())
+    assert ((C.double() - Ad @ Bd).abs() <= bound).all()
