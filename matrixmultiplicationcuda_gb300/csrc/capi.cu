@@ -492,6 +492,12 @@ spmm_status spmm_bcsr_mm_nnzb(const spmm_bcsr_desc* A, long long nnzb, const spm
         r.cfg.n_tile = 256;
         r.cfg.stages = 0;
         r.cfg.schedule = 1;
+      } else if (e4m3 && nnzb >= 0) {
+        // Lines where groups begin to pay: 16 rows of 3 to 8 blocks take 0.92 of the
+        // time in groups, 64 rows of 3 to 8 1.00; 32 rows of 5 to 14 with several CTAs
+        // on an SM 1.04 (174 rows of 6, N 400: 8.1, 6.9 us in single blocks), else 0.89.
+        const bool full = (long long)(A->M / 32) * ((N + 127) / 128) > sm_count();
+        r.single_blocks = (double)nnzb * A->bR < (A->bR == 16 ? 2.5 : A->bR == 32 && full ? 14 : 5.5) * A->M;
       }
     } else {
       r.cfg.kernel = A->bR == 64 && !e4m3 ? 2 : 1;

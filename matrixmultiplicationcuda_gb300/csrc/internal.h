@@ -80,6 +80,8 @@ struct LaunchRequest {
   // e4m3 converted to fp16 on the way into shared memory (any block scale),
   // in place of the block-scaled MMA (powers of two)
   bool convert = false;
+  // e4m3 on mma.sync: ring slots of one block instead of four (short rows)
+  bool single_blocks = false;
   // planned product (kernel 2): the item list, split-row pairs and their
   // counters (see spmm_bcsr_plan_create)
   const int4* items = nullptr;

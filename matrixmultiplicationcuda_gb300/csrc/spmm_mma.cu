@@ -12,7 +12,7 @@ namespace {
 using KernelFn = void (*)(const CUtensorMap, const CUtensorMap, const MmaParams);
 
 struct Entry {
-  int br, mode, nt, stages, wm, wn;
+  int br, mode, nt, stages, group;
   KernelFn fn;
   size_t smem;
   int threads;
@@ -23,8 +23,7 @@ struct Entry {
         MODE,                                                                      \
         NT,                                                                        \
         ST,                                                                        \
-        WM,                                                                        \
-        WN,                                                                        \
+        GROUP,                                                                     \
         &k_bcsr_mma<BR, NT, WM, WN, RING, GROUP, MODE>,                            \
         MmaCfg<BR, NT, WM, WN, RING, GROUP, MODE>::kSmem,                          \
         MmaCfg<BR, NT, WM, WN, RING, GROUP, MODE>::kThreads}
@@ -40,7 +39,9 @@ struct Entry {
 // than a group leave part of its slots empty (two blocks a row, 16384 x 2048, N
 // 1024: 16.1 us, 16.8 with groups). e4m3's blocks are half as large, so its
 // rings hold eight at the same occupancy (16 rows, 8192^2, 10 %, N 1024: 119
-// us with single blocks, 102; log-normal rows, 5 %, N 512: 77, 58).
+// us with single blocks, 102; log-normal rows, 5 %, N 512: 77, 58). Rows known to
+// be short take single blocks there too (12160 x 3872, 32 rows, four blocks a row,
+// N 144: 4.9 us, 5.9 with groups; 4416 x 736, 64 rows, two, N 1008: 6.0, 6.7).
 // The configuration space the tuner sweeps (block height x column tile x depth).
 #define SPMM_MMA_SHAPES(MODE)                                                      \
   SPMM_MMA_ENTRY(16, 64, 1, 4, 4, MODE), SPMM_MMA_ENTRY(16, 128, 1, 4, 4, MODE),    \
@@ -58,6 +59,11 @@ const Entry kEntries[] = {
     SPMM_MMA_ENTRY(32, 128, 2, 2, 4, MODE_SPLIT),
     SPMM_MMA_ENTRY(64, 128, 2, 2, 4, MODE_SPLIT),
     SPMM_MMA_ENTRY(64, 64, 4, 1, 4, MODE_SPLIT),
+    // e4m3 in single blocks (LaunchRequest::single_blocks)
+    SPMM_MMA_ENTRY_AS(16, 128, 1, 4, 4, 4, 1, MODE_E4M3),
+    SPMM_MMA_ENTRY_AS(16, 256, 1, 4, 4, 4, 1, MODE_E4M3),
+    SPMM_MMA_ENTRY_AS(32, 128, 2, 2, 4, 4, 1, MODE_E4M3),
+    SPMM_MMA_ENTRY_AS(64, 128, 2, 2, 4, 4, 1, MODE_E4M3),
     SPMM_MMA_ENTRY_AS(16, 128, 1, 4, 4, 8, 4, MODE_E4M3),
     SPMM_MMA_ENTRY_AS(16, 256, 1, 4, 4, 8, 4, MODE_E4M3),
     SPMM_MMA_ENTRY_AS(32, 128, 2, 2, 4, 8, 4, MODE_E4M3),
@@ -84,10 +90,11 @@ int default_nt(int br, int mode, int N) {
   return N >= 128 ? 128 : 64;
 }
 
-const Entry* find_entry(int br, int mode, int nt, int stages) {
+const Entry* find_entry(int br, int mode, int nt, int stages, bool single_blocks = false) {
   const Entry* best = nullptr;
   for (const Entry& e : kEntries) {
     if (e.br != br || e.mode != mode || e.nt != nt) continue;
+    if (mode == MODE_E4M3 && (e.group == 1) != single_blocks) continue;
     if (stages > 0 && e.stages != stages) continue;
     if (!best || (stages <= 0 && e.stages == 4)) best = &e;
   }
@@ -114,7 +121,7 @@ spmm_status launch_mma(const LaunchRequest& r) {
   const int mode = mode_of(A.dtype);
   if (mode < 0) return fail(SPMM_ERR_INVALID_ARG, "unknown dtype");
   const int nt = r.cfg.n_tile > 0 ? r.cfg.n_tile : default_nt(A.bR, mode, r.N);
-  const Entry* e = find_entry(A.bR, mode, nt, r.cfg.stages);
+  const Entry* e = find_entry(A.bR, mode, nt, r.cfg.stages, r.single_blocks);
   if (!e)
     return fail(SPMM_ERR_UNSUPPORTED, "no mma.sync kernel for bR=" + std::to_string(A.bR) +
                                           " n_tile=" + std::to_string(nt) +

@@ -158,3 +158,32 @@ def test_converted_product_at_the_rule(dev, bR, items, K, N, pad):
     terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
     bound = terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs())
     assert ((C.double() - Ad @ Bd).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("bR,N", [(16, 144), (16, 4096), (32, 128), (64, 272)])
+@pytest.mark.parametrize("per_row", [0, 1, 2, 5])
+def test_short_rows(dev, bR, N, per_row):
+    """Rows of at most five blocks, which mma.sync takes one by one; bound as above."""
+    MB, KB = 160, 12
+    rng = np.random.default_rng(N + per_row)
+    keep = np.zeros((MB, KB), bool)
+    for r in range(MB):
+        keep[r, rng.choice(KB, min(KB, max(0, per_row + int(r == 9) * 7 - int(r == 4))), replace=False)] = True
+    g = torch.Generator(device=dev).manual_seed(N + bR)
+    n = int(keep.sum())
+    vals = torch.randint(0, 0x7f, (n, bR, 16), generator=g, device=dev, dtype=torch.uint8)
+    sc = torch.rand(n, generator=g, device=dev) * 0.02 + 1e-4
+    t = lambda a: torch.from_numpy(np.ascontiguousarray(a.astype(np.int32))).to(dev)
+    A = m.BCSR(MB * bR, KB * 16, bR, 16, t(np.concatenate([[0], np.cumsum(keep.sum(1))])), t(np.nonzero(keep)[1]),
+               vals.view(-1), m.DType.E4M3, None, sc)
+    B = torch.randint(0, 0x7f, (KB * 16, N), generator=g, device=dev, dtype=torch.uint8)
+    C = torch.full((MB * bR, N), float("nan"), device=dev)
+    m.spmm(A, B, C=C)
+    m.device_error_check()
+    Ad = torch.zeros(MB, KB, bR, 16, dtype=torch.float64, device=dev)
+    Ad[torch.from_numpy(keep).to(dev)] = (vals.view(torch.float8_e4m3fn).float() * sc[:, None, None]).half().double()
+    Ad = Ad.permute(0, 2, 1, 3).reshape(MB * bR, KB * 16)
+    Bd = B.view(torch.float8_e4m3fn).double()
+    terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
+    bound = terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs())
+    assert ((C.double() - Ad @ Bd).abs() <= bound).all()
