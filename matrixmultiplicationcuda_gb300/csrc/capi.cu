@@ -557,10 +557,10 @@ spmm_status spmm_hcsr_mm(const spmm_bcsr_desc* A, const spmm_csr_desc* R, const 
   r.stream = static_cast<cudaStream_t>(stream);
   // The CSR part in a launch of its own runs on every warp of an SM; in the
   // epilogue it has eight, whose B loads wait for L2. us, two launches against
-  // the fused one: 4096^2, 10 % blocks, 2 % entries, N 1024: 70.8, 131; 0.5 %
-  // entries, N 512: 21.6, 29.4; 1024^2, N 1024: 13.8, 16.0; 4096^2, N 64: 26.7,
-  // 37.4; 5 % blocks, 0.1 % entries, N 128: 11.4, 11.4. Two launches cost the
-  // host more than the smallest products take: 1024^2, N 64: 11.4, 8.5.
+  // the fused one: 4096^2, 10 % blocks, 2 % entries, N 1024: 68.8, 106; 0.5 %
+  // entries, N 512: 24.1, 27.6; 1024^2, N 1024: 14.7, 15.0; 4096^2, N 64: 30.3,
+  // 31.8; 5 % blocks, 0.1 % entries, N 128: 11.1, 12.0. Two launches cost a calling
+  // loop more than the smallest products take: 256 x 288, N 2400: 11.2, 9.1.
   if (!cfg && (long long)A->M * N >= 1 << 18 && N <= 65535 * 256) {
     const spmm_status st = launch_tc(r);
     return st != SPMM_OK ? st : launch_csr_add(*R, *B, N, C, ldc, r.stream);

@@ -4,11 +4,12 @@
 //
 // One warp per (row, 256-column slice), through the row-slice routine of
 // csr.cuh: every lane owns 8 consecutive output columns, B rows are read as
-// 512-byte warp loads with 8 entries in flight, and the row's results leave as
-// two 16-byte streaming stores per lane. Bound by L2's latency: 4096^2, 2 % (302k
-// entries), N 1024, 618 MB of B rows: 50 us, 54 with 4 entries in flight and
-// their indices read just before them; a 4096 x 1024 matrix of 0.2 % entries,
-// which ends in the remainders of short rows, 6.1 us from 10.2.
+// 512-byte warp loads with 4 entries in flight, and the row's results leave as
+// two 16-byte streaming stores per lane. Bound by L2's latency, so by the warps on
+// an SM: with 8 entries in flight (80 registers, three CTAs an SM instead of five)
+// 7232 x 1232, 0.06 %, N 128 takes 4.6 us where it takes 4.0; 4096^2, 2 % (302k
+// entries), N 1024, 618 MB of B rows: 48 us, 50 with 8, 54 with 4 and their indices
+// read just before them.
 #include <cuda_fp16.h>
 #include "csr.cuh"
 #include "internal.h"
@@ -37,7 +38,7 @@ __global__ void __launch_bounds__(32 * kCsrWarps)
   const int n = blockIdx.y * 256 + lane * 8;
   const bool valid = n < N;   // N is a multiple of 8
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  csr_row_slice<8>(col_idx, vals, B, ldb, e0, e1, n, valid, acc);
+  csr_row_slice<4>(col_idx, vals, B, ldb, e0, e1, n, valid, acc);
   if (valid) {
     float* c = C + (long long)row * ldc + n;
     if constexpr (ADD) {

@@ -8,6 +8,7 @@
 #pragma once
 #include <cuda_fp16.h>
 #include <cstdint>
+#include <type_traits>
 
 namespace spmm {
 
@@ -28,12 +29,12 @@ __device__ __forceinline__ void fma8(float (&acc)[8], float a, uint4 b) {
 // waits for no index, and the last entries of a row load together like any
 // others (one by one, with their indices read first, a row's last U - 1 entries
 // took as long as 2 U (U - 1) others).
-template <int U>
+template <int U>   // 4 or 8
 __device__ __forceinline__ void csr_row_slice(const int* __restrict__ col_idx, const __half* __restrict__ vals,
                                               const __half* __restrict__ B, long long ldb, int e0, int e1, int n,
                                               bool valid, float (&acc)[8]) {
   const int lane = threadIdx.x & 31;
-  const __half* src = B + (valid ? n : 0);
+  const __half* src = B + (valid ? n : n - 8 * lane);   // past N: the slice's first column
   int next_k = 0;
   __half next_a = __float2half(0.f);
   if (e0 + lane < e1) {
@@ -47,20 +48,35 @@ __device__ __forceinline__ void csr_row_slice(const int* __restrict__ col_idx, c
       next_k = __ldg(col_idx + base + 32 + lane);
       next_a = __ldg(vals + base + 32 + lane);
     }
-    for (int i = 0; i < cnt; i += U) {
-      // (no condition on a load: past the last entry its row again, past N column 0)
-      uint4 b[U];
+    // V entries from i on, of which the first n are there (no condition on a load:
+    // past the last entry its row again)
+    auto entries = [&](auto count, int i, int n) {
+      constexpr int V = decltype(count)::value;
+      uint4 b[V];
 #pragma unroll
-      for (int t = 0; t < U; ++t) {
-        const unsigned k = (unsigned)__shfl_sync(0xffffffffu, ks, min(i + t, cnt - 1));
+      for (int t = 0; t < V; ++t) {
+        const unsigned k = (unsigned)__shfl_sync(0xffffffffu, ks, i + min(t, n - 1));
         b[t] = __ldg(reinterpret_cast<const uint4*>(src + (unsigned long long)k * (unsigned)ldb));
       }
 #pragma unroll
-      for (int t = 0; t < U; ++t) {
+      for (int t = 0; t < V; ++t) {
         const float a = __shfl_sync(0xffffffffu, as, (i + t) & 31);
-        if (i + t < cnt) fma8(acc, a, b[t]);
+        if (t < n) fma8(acc, a, b[t]);
       }
-    }
+    };
+    int i = 0;
+    for (; cnt - i >= U; i += U) entries(std::integral_constant<int, U>{}, i, U);
+    // the rest in the smallest step that holds it: a row of one entry in eight loads
+    // took 4.3 us where one takes 3.2 (5056 x 832, 0.1 %, N 64)
+    const int rest = cnt - i;
+    if (rest > U / 2)
+      entries(std::integral_constant<int, U>{}, i, rest);
+    else if (U > 4 && rest > 2)
+      entries(std::integral_constant<int, U / 2>{}, i, rest);
+    else if (rest == 2)
+      entries(std::integral_constant<int, 2>{}, i, 2);
+    else if (rest == 1)
+      entries(std::integral_constant<int, 1>{}, i, 1);
   }
 }
 
