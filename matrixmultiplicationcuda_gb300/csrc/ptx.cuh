@@ -144,6 +144,12 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
+// 16 bytes where `on`, else nothing
+__device__ __forceinline__ void cp_async16_if(uint32_t dst, const void* src, bool on) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p cp.async.cg.shared.global [%0], [%1], 16;\n\t}" ::"r"(dst),
+               "l"(src), "r"((int)on)
+               : "memory");
+}
 // 16 bytes, or 16 zero bytes (src is not read then)
 __device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool read) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(read ? 16 : 0) : "memory");
