@@ -245,7 +245,6 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
   }
 }
 
-// Two e4m3 values in the low 16 bits -> f16x2 (exact: e4m3 is a subset of fp16).
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t src) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
@@ -260,6 +259,7 @@ __device__ __forceinline__ void st_shared_v4(uint32_t dst, uint4 v) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                : "memory");
 }
+// Two e4m3 values in the low 16 bits -> f16x2 (exact: e4m3 is a subset of fp16).
 __device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t v16) {
   uint32_t r;
   asm("{\n\t.reg .b16 t;\n\tmov.b32 {t, _}, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, t;\n\t}"

@@ -62,7 +62,6 @@ struct TcParams {
   int panel3d;      // B panel loaded by one 3-D copy (N % 64 == 0)
   int dynamic;      // later items: 1 = the grid's pending blocks (one block per item), 0 = the queue or a static stride
   unsigned* queue;  // a plan's queue: [0] next item, [1] CTAs done; NULL = none
-  int claim_ahead;  // dynamic, queue: claim the next item when this many groups of the current one are left to copy
   int inputs_ready; // no kernel earlier on the stream writes A or B (see the dependency wait below)
   int split;        // items per (block row, column tile); > 1: partial sums added into C
   // hybrid (BCSR + CSR): the CSR part's entries are added in the epilogue
@@ -206,7 +205,6 @@ struct TcCfg {
 
 constexpr int kTcThreads = 352;   // 11 warps
 
-
 template <int BR, int NT, int STAGES, int MODE, int ACC, int G, int FEED = kFeedTma>
 __global__ void __launch_bounds__(kTcThreads, 2)
     k_bcsr_tc(const __grid_constant__ CUtensorMap tmA1, const __grid_constant__ CUtensorMap tmAg,
@@ -323,10 +321,11 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 
   if (warp == 0) {
     // ------------------------------ lead producer ----------------------------------
-    // Takes items (work queue or static stride), publishes them through the item
-    // ring (-1 ends the stream), and for each group of the item's blocks claims
-    // the ring slot, expects the group's bytes on its full barrier and copies the
-    // A blocks. The B issuers copy the group's B panels into the same slot.
+    // Takes items (the grid's pending blocks, a plan's queue or a static stride),
+    // publishes them through the item ring (-1 ends the stream), and for each group
+    // of the item's blocks claims the ring slot, expects the group's bytes on its
+    // full barrier and copies the A blocks. The B issuers copy the group's B panels
+    // into the same slot.
     if (lane == 0) {
       if constexpr (!CONVERT) {
         tma_prefetch_desc(&tmAg);
@@ -378,11 +377,11 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       };
       // Items after the first: static striding (blockIdx.x + k * gridDim.x),
       // blocks of the grid that have not started, or tickets from a plan's work
-      // queue offset by the grid size. A claim is made late, when claim_ahead
-      // groups of the current item are left to copy (< 0: as the item starts),
-      // so that a CTA running faster (lighter items, or an SM it no longer
-      // shares) takes more of the items still unclaimed; it is issued one group
-      // before its result is used, and the item goes into the ring at once.
+      // queue offset by the grid size. A claim is made late, when kClaimAhead
+      // groups of the current item are left to copy, so that a CTA running faster
+      // (lighter items, or an SM it no longer shares) takes more of the items still
+      // unclaimed; it is issued one group before its result is used, and the item
+      // goes into the ring at once.
       // (Claiming two items ahead, with the block ranges and column indices of
       // the next one loaded early, made short rows no faster and cost every
       // other shape 5-15 %: the issuing warps' instructions per group count.)
@@ -399,7 +398,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       auto copy_items = [&](auto way) {
         constexpr int kWay = decltype(way)::value;   // 1 = pending blocks, 0 = queue or stride, -1 = as p.dynamic says
         const bool dynamic = kWay >= 0 ? kWay != 0 : p.dynamic != 0;
-        const bool late = (dynamic || p.queue != nullptr) && p.claim_ahead >= 0 && !no_more;
+        const bool late = (dynamic || p.queue != nullptr) && !no_more;
+        constexpr int kClaimAhead = STAGES - 1;   // (the B issuers' waits count on it, see there)
         uint32_t claims = 0;
         auto claim = [&]() -> unsigned {
           if (!dynamic) {
@@ -444,9 +444,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
           unsigned ticket = 0;
           if (!late) {
             // the next item's indices load now and are used once this item is copied
-            nitem = no_more ? -1
-                    : dynamic || p.queue ? claimed_item(claim())
-                                           : (item + (int)gridDim.x < p.n_items ? item + (int)gridDim.x : -1);
+            nitem = !no_more && item + (int)gridDim.x < p.n_items ? item + (int)gridDim.x : -1;
             range(nitem, &nstart, &nend, &ntile);
           }
           const int ngroups = (end - start + G - 1) / G;
@@ -466,7 +464,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
                 range(nitem, &nstart, &nend, &ntile);
                 publish(it + 1, nitem, nstart, nend, ntile);
                 if (failed) break;
-              } else if (ngroups - gi <= p.claim_ahead + 1) {
+              } else if (ngroups - gi <= kClaimAhead + 1) {
                 ticket = claim();
                 claimed = true;
               }
@@ -770,7 +768,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             // order, so the wait in an issuer's previous group covers it as long as
             // that group is at most STAGES groups back: issuers skip only an item's
             // last, partial group, and the lead publishes an item once the group
-            // 2 * STAGES before its first has been consumed (claim_ahead = STAGES - 1).
+            // 2 * STAGES before its first has been consumed (kClaimAhead).
             // (Rotating the block-to-issuer map over groups of fewer than four
             // blocks breaks this and was measured to corrupt a slot.) With gather
             // blocks every issuer arrives in every group, so every one waits.
@@ -1338,7 +1336,6 @@ spmm_status launch_tc(const LaunchRequest& r) {
   p.timeout_ns = wait_limit_ns();
   p.err = r.err_word ? r.err_word : device_error_word();
   p.panel3d = panel3d;
-  p.claim_ahead = e->stages - 1;
   p.inputs_ready = r.inputs_ready ? 1 : 0;
   p.csr_row_ptr = r.csr ? r.csr->row_ptr : nullptr;
   p.csr_col_idx = r.csr ? r.csr->col_idx : nullptr;
@@ -1393,9 +1390,9 @@ spmm_status launch_tc(const LaunchRequest& r) {
   if (std::getenv("SPMM_DEBUG"))
     std::fprintf(stderr,
                  "[spmm] tcgen05 bR=%d nt=%d stages=%d acc=%d group=%d smem=%zu tmem=%d per_sm=%d grid=%lld "
-                 "items=%d panel3d=%d dynamic=%d queue=%d claim_ahead=%d inputs_ready=%d split=%d\n",
+                 "items=%d panel3d=%d dynamic=%d queue=%d inputs_ready=%d split=%d\n",
                  A.bR, nt, e->stages, e->acc, e->group, smem, e->tmem_cols, per_sm, grid, p.n_items, panel3d,
-                 p.dynamic, p.queue != nullptr, p.claim_ahead, p.inputs_ready, p.split);
+                 p.dynamic, p.queue != nullptr, p.inputs_ready, p.split);
   SPMM_CUDA_TRY(launch_kernel(e->fn, dim3((unsigned)grid), dim3(kTcThreads), smem, r.stream, tmA1, tmAg, tmAlo1,
                               tmAlog, tmB, tmBlo, p));
   return SPMM_OK;

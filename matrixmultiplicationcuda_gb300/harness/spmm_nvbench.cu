@@ -160,12 +160,12 @@ std::string config_name(const spmm_config* c) {
   if (c->kernel == 1)
     std::snprintf(b, sizeof(b), "mma nt%d st%d", c->n_tile, c->stages);
   else if (c->kernel == 3)
-    std::snprintf(b, sizeof(b), "tc64 nt%d %s", c->n_tile, c->schedule ? "queue" : "static");
+    std::snprintf(b, sizeof(b), "tc64 nt%d %s", c->n_tile, c->schedule ? "dynamic" : "static");
   else if (c->schedule == 2)
     std::snprintf(b, sizeof(b), "plan tc nt%d st%d acc%d", c->n_tile, c->stages, c->acc_buffers);
   else
     std::snprintf(b, sizeof(b), "tc nt%d st%d acc%d %s split%d", c->n_tile, c->stages, c->acc_buffers,
-                  c->schedule ? "queue" : "static", c->split_k > 1 ? c->split_k : 1);
+                  c->schedule ? "dynamic" : "static", c->split_k > 1 ? c->split_k : 1);
   return b;
 }
 
