@@ -742,6 +742,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         }
         // gather blocks: lane r < 16 has B row r of gather block next_g (< 0: none)
         [[maybe_unused]] int next_g = -1, next_rows = 0;
+        [[maybe_unused]] const bool full_tile = nt * NT + NT <= p.N;
         for (int base = start; base < end && !failed; base += 32) {
           const int cnt = min(32, end - base);
           const int cur = mycol;
@@ -826,7 +827,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
                     const bool on = n0 < p.N;
                     const __half* src = p.Bh + (on ? n0 : 0);
                     const uint32_t dst = smem_u32(b_dst + (c >> 3) * Cfg::kBoxBytes), sw = (uint32_t)(c & 7) << 4;
-                    if (whole && nt * NT + NT <= p.N) {
+                    if (whole && full_tile) {
 #pragma unroll
                       for (int r = 0; r < 16; ++r) {
                         const unsigned row = (unsigned)__shfl_sync(0xffffffffu, rows, r);
