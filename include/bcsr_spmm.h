@@ -94,7 +94,9 @@ const char* spmm_last_error(void);
  * E4M3 needs multiples of 16. cfg may be NULL.
  * E4M3 with kernel 0 runs the mma.sync pipeline or, for 32- and 64-row blocks
  * and longer rows when the number of stored blocks is known (see below), the
- * tcgen05 pipeline on e4m3 converted to fp16; both take any fp32 block scale.
+ * tcgen05 pipeline on e4m3 converted to fp16; both take any fp32 block scale
+ * whose products with the block's values fp16 holds: value x scale is rounded to
+ * fp16, so above 65504 C gets infinities, and below 2^-14 precision is lost.
  * Kernel 2 runs the tcgen05 block-scaled kernels (kind::mxf8f6f4):
  * every block scale must be a positive normal power of two, as spmm_quantize
  * makes them (another scale raises a flag spmm_device_error_check reports);

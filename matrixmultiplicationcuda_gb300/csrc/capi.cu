@@ -326,7 +326,8 @@ namespace spmm {
 //     on: 8192^2, 10 a row, N 1024: 20.9, 22.0. Its tile is 256 columns wide, so
 //     the last one has to be at least half used.
 //   e4m3: mma.sync or, where converts_e4m3 says so, the tcgen05 pipeline with
-//     e4m3 converted to fp16; both take any block scale (the block-scaled MMA,
+//     e4m3 converted to fp16; both take any block scale whose products with the
+//     block's values fp16 holds (the block-scaled MMA,
 //     which a caller may ask for, is faster but needs powers of two). 16 rows and
 //     2048 items or more: mma.sync's 256-column tile (8192^2, 10 %, N 1024: 80
 //     against 102 for 128 columns; 2 % and log-normal rows, N 2048: 48 against 59;

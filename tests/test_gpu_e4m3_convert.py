@@ -187,3 +187,28 @@ def test_short_rows(dev, bR, N, per_row):
     terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
     bound = terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs())
     assert ((C.double() - Ad @ Bd).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("MB,N", [(24, 128), (230, 512)])     # mma.sync, converted
+def test_scales_at_the_ends_of_fp16(dev, MB, N):
+    """Block scales that take the largest e4m3 value to fp16's largest (146.2 x 448),
+    and ones whose products are subnormal there. Against scaled values in FP64: each
+    is off by half a step of fp16, 2^-11 of it or 2^-25, and the sums as above."""
+    bR, KB = 64, 24
+    g = torch.Generator(device=dev).manual_seed(N)
+    n = MB * KB
+    vals = torch.randint(0, 0x7f, (n, bR, 16), generator=g, device=dev, dtype=torch.uint8)
+    vals ^= torch.randint(0, 2, (n, bR, 16), generator=g, device=dev, dtype=torch.uint8) << 7
+    sc = torch.where(torch.rand(n, generator=g, device=dev) < 0.5, 146.2, 2.0 ** -20)
+    i = lambda t: t.to(torch.int32).contiguous()
+    A = m.BCSR(MB * bR, KB * 16, bR, 16, i(torch.arange(MB + 1, device=dev) * KB), i(torch.arange(KB, device=dev).repeat(MB)),
+               vals.view(-1), m.DType.E4M3, None, sc)
+    B = torch.randint(0, 0x7f, (KB * 16, N), generator=g, device=dev, dtype=torch.uint8)
+    C = m.spmm(A, B)
+    m.device_error_check()
+    Ad = (vals.view(torch.float8_e4m3fn).double() * sc.double()[:, None, None]).view(MB, KB, bR, 16)
+    Ad = Ad.permute(0, 2, 1, 3).reshape(MB * bR, KB * 16)
+    Bd = B.view(torch.float8_e4m3fn).double()
+    off = torch.clamp(Ad.abs() * 2.0 ** -11, min=2.0 ** -25)
+    bound = off @ Bd.abs() + 16 * KB * 2.0 ** -23 * ((Ad.abs() + off) @ Bd.abs())
+    assert ((C.double() - Ad @ Bd).abs() <= bound).all()
