@@ -282,12 +282,12 @@ spmm_status spmm_device_error_check(void* stream) {
 namespace spmm {
 
 // What a product with no configuration runs, from its sizes and (nnzb >= 0) the
-// number of stored blocks. The lines stand where neither side of one was more
-// than 5 % slower than a single fixed kernel (the 128- or 256-column tcgen05
-// kernel for 64 rows, mma.sync with single blocks for 16 and 32), over 2000
-// products (M to 16384, K 256 to 16384, N 40 to 4096, 0.5 to 300 blocks a row;
-// even, random and log-normal rows; replayed ten at a time on one GB300). items:
-// block rows x 256-column tiles. Times in us, the line's two sides:
+// number of stored blocks. The lines stand where neither side of one was much
+// slower than a single fixed kernel (the 128- or 256-column tcgen05 kernel for 64
+// rows, mma.sync with single blocks for 16 and 32): at most 9 %, over 2500 products
+// (M to 16384, K 256 to 16384, N 40 to 4096, 0.5 to 300 blocks a row; even, random
+// and log-normal rows; replayed ten at a time on one GB300). items: block rows x
+// 256-column tiles. Times in us, the line's two sides:
 //   64-row blocks, fp16 and bf16:
 //     - next to nothing to do (known): mma.sync. 43 rows of one block, N 104: 2.5
 //       (64-row pipeline 4.3, tc128 4.8). Not for long rows, whose blocks one CTA
@@ -327,13 +327,13 @@ namespace spmm {
 //     the last one has to be at least half used.
 //   e4m3: mma.sync or, where converts_e4m3 says so, the tcgen05 pipeline with
 //     e4m3 converted to fp16; both take any block scale whose products with the
-//     block's values fp16 holds (the block-scaled MMA,
-//     which a caller may ask for, is faster but needs powers of two). 16 rows and
-//     2048 items or more: mma.sync's 256-column tile (8192^2, 10 %, N 1024: 80
-//     against 102 for 128 columns; 2 % and log-normal rows, N 2048: 48 against 59;
-//     16384 x 4096, 2 %, N 512: 14.0 against 16.2). With fewer, 128 columns
-//     spread long rows further (16384 x 4096, log-normal, N 256: 16.4 against
-//     19.0), as where half of the last 256 would be empty (N 272: 13.2, 14.2).
+//     block's values fp16 holds (the block-scaled MMA, which a caller may ask for,
+//     is faster but needs powers of two). 16 rows and 2048 items or more:
+//     mma.sync's 256-column tile (8192^2, 10 %, N 1024: 80 against 102 for 128
+//     columns; 2 % and log-normal rows, N 2048: 48 against 59; 16384 x 4096, 2 %, N
+//     512: 14.0 against 16.2). With fewer, 128 columns spread long rows further
+//     (16384 x 4096, log-normal, N 256: 16.4 against 19.0), as where half of the
+//     last 256 would be empty (N 272: 13.2, 14.2).
 spmm_config default_config(int bR, spmm_dtype dtype, int M, int N, long long nnzb) {
   spmm_config c;
   std::memset(&c, 0, sizeof(c));
