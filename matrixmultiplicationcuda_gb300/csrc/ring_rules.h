@@ -24,13 +24,13 @@ constexpr int kBIssuers = 4;    // B-issuing warps
 constexpr int kConvertFullArrivals = kBIssuers + 1;
 
 // Converted e4m3: a B issuer copies groups ahead of those it converts, across
-// items. Whether it may wait for an entry of the item ring that lies `ahead`
-// entries after the one whose group it has to convert next. The lead publishes
-// entry e once entry e - kItemRing has been read, and the MMA threads and the
-// epilogue read that one after finishing entry e - kItemRing - 1; an issuer that
-// waits for e with a group of that entry or an older one unconverted waits for
-// itself (items without blocks bring it there: they hold no group).
-SPMM_RULE bool may_wait_for_entry(uint32_t ahead) { return ahead <= (uint32_t)kItemRing; }
+// items. Whether one that has converted `converted` groups may wait for an entry
+// of the item ring, `first` being the first group of the entry kItemRing before
+// it. The lead publishes an entry once that one has been read, and the MMA threads
+// and the epilogue read it after finishing the entry before it; an issuer that
+// waits with a group of that entry or an older one unconverted waits for itself
+// (items without blocks bring it there: they hold no group).
+SPMM_RULE bool may_wait_for_entry(uint32_t converted, uint32_t first) { return (int32_t)(converted - first) >= 0; }
 
 }  // namespace spmm
 #undef SPMM_RULE

@@ -570,7 +570,6 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       constexpr int kDepth = Cfg::kDepth, kPer = kBIssuers / G, kRows = 16 / kPer, kARows = BR / kPer;
       constexpr int kCopies = Cfg::kCopies;
       static_assert(!CONVERT || (NT == 256 && kARows <= 32 && kBIssuers % G == 0), "the lane maps below");
-      static_assert(!CONVERT || (kDepth >= 2 && kDepth <= 3), "the waits for a group's copies below");
       const int myb = bidx / kPer, part = bidx % kPer;
       // Lane: 16 columns (a 16-byte chunk c) of rows r0, r0 + 2, ...: eight lanes
       // hold four chunks of two rows, whose fp16 stores fall on all banks.
@@ -583,15 +582,17 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       const uint32_t raw0 = smem_u32(smem) + STAGES * Cfg::kStage + bidx * (kDepth * Cfg::kRawGroup);
       // the copying end of the stream
       uint32_t it = 0, copied = 0, gs = 0;    // next entry of the item ring; groups copied, converted
-      uint32_t has = 0, entries = 0;          // bit g % 32: group g holds a block of this issuer; byte g % 4: its entry
+      uint32_t has = 0;                       // bit g % 32: group g holds a block of this issuer
+      uint32_t first = 0;                     // lane e % kItemRing: first group of entry e
       int j0 = 0, end = 0, base = 0, cols = 0, next_cols = 0;   // next group; lane's column indices from base, base + 32
       const uint8_t* bcol = bsrc;
       bool done = false;
-      // One more group, if there is one (its copies are one cp.async group). False
-      // at the end of the items, and where the next item may not be waited for yet.
+      // The copies of one more group, as one cp.async group. False at the end of the
+      // items, and where the next item may not be waited for yet.
       auto copy_group = [&]() -> bool {
         while (!done && j0 >= end) {
-          if (copied != gs && !may_wait_for_entry((it - (entries >> (8 * (gs & 3)))) & 255u)) return false;
+          if (!may_wait_for_entry(gs, __shfl_sync(0xffffffffu, first, it % kItemRing))) return false;
+          if (lane == it % kItemRing) first = copied;
           int item = -1, start = 0, e = 0, nt = 0, ok = 1;
           if (lane == 0) ok = read_item(it, &item, &start, &e, 4u, &nt) ? 1 : 0;
           ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -614,8 +615,6 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         }
         const int j = j0 + myb;
         has &= ~(1u << (copied & 31));
-        const uint32_t sh = 8 * (copied & 3);
-        entries = (entries & ~(255u << sh)) | (((it - 1) & 255u) << sh);
         if (j < end) {
           has |= 1u << (copied & 31);
           const int col = __shfl_sync(0xffffffffu, cols, j - base);
@@ -639,12 +638,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
       auto half8 = [](uint32_t x, uint32_t y) {   // 8 e4m3 -> 8 fp16
         return make_uint4(e4m3x2_to_f16x2(x), e4m3x2_to_f16x2(x >> 16), e4m3x2_to_f16x2(y), e4m3x2_to_f16x2(y >> 16));
       };
-#pragma unroll 1
-      for (;; ++gs) {
-#pragma unroll 1
-        while (copied - gs < (uint32_t)kDepth && copy_group()) {
-        }
-        if (copied == gs) break;   // (with nothing left to convert the next item is always waited for)
+      // Converts group gs into its slot. False if the wait for the slot gave up.
+      auto convert_group = [&]() -> bool {
         const int s = (int)(gs % STAGES);
         int bad = 0;
         if (lane == 0 && gs >= (uint32_t)STAGES &&
@@ -652,12 +647,11 @@ __global__ void __launch_bounds__(kTcThreads, 2)
           atomicOr(p.err, 4u);
           bad = 1;
         }
-        if (__shfl_sync(0xffffffffu, bad, 0)) break;
-        // group gs has landed: all but the groups copied after it
+        if (__shfl_sync(0xffffffffu, bad, 0)) return false;
+        // group gs has landed (fewer follow it after the last group and while the
+        // next item may not be waited for)
         if (copied - gs == (uint32_t)kDepth)
           cp_async_wait_group<kDepth - 1>();
-        else if (copied - gs == 2)
-          cp_async_wait_group<1>();
         else
           cp_async_wait_group<0>();
         __syncwarp();   // the slot is free for every lane; lane 0's copy of the scale has landed
@@ -701,6 +695,24 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(full0 + 8 * s);
+        return true;
+      };
+      // Copies ahead until as many groups as the ring is deep wait to be converted,
+      // then converts one and copies one while that stays so. (With every group
+      // converted the next item is always waited for: no group left means the end.)
+      bool ok = true;
+      while (ok) {
+#pragma unroll 1
+        while (copied - gs < (uint32_t)kDepth && copy_group()) {
+        }
+        if (copied == gs) break;
+#pragma unroll 1
+        do {
+          ok = convert_group();
+          if (!ok) break;
+          ++gs;
+          copy_group();
+        } while (copied - gs == (uint32_t)kDepth);
       }
       cp_async_wait_all();
     };

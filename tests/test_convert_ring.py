@@ -21,7 +21,7 @@ def rules(tmp_path_factory):
     src.write_text('#include "ring_rules.h"\nextern "C" {\nint entries() { return spmm::kItemRing; }\n'
                    'int issuers() { return spmm::kBIssuers; }\n'
                    'int arrivals() { return spmm::kConvertFullArrivals; }\n'
-                   'int may_wait(unsigned ahead) { return spmm::may_wait_for_entry(ahead); }\n}\n')
+                   'int may_wait(unsigned converted, unsigned first) { return spmm::may_wait_for_entry(converted, first); }\n}\n')
     so = d / "rules.so"
     subprocess.run(["g++", "-std=c++17", "-shared", "-fPIC", "-I" + CSRC, str(src), "-o", str(so)], check=True)
     return ctypes.CDLL(str(so))
@@ -101,19 +101,21 @@ class Cta:
                 gs += 1
 
     def issuer(self, me):
-        it = left = gs = 0
-        done, ahead = False, []   # entries of the groups copied and not yet converted
+        it = left = copied = gs = 0
+        done, first = False, [0] * self.Q   # first group of each entry of the item ring
         while True:
-            while len(ahead) < self.stages:
-                while not done and left == 0 and (not ahead or self.may_wait(it - ahead[0])):
+            while copied - gs < self.stages:
+                while not done and left == 0 and self.may_wait(gs, first[it % self.Q]):
+                    first[it % self.Q] = copied
                     left = yield from self.read(it)
                     it += 1
                     done = left < 0
                 if done or left == 0:
                     break
                 left -= 1
-                ahead.append(it - 1)
-            if not ahead:
+                copied += 1
+            if copied == gs:
+                assert done
                 return
             s = gs % self.stages
             if gs >= self.stages:
@@ -122,7 +124,6 @@ class Cta:
             self.slot[s][me] = gs
             self.full[s].arrive()
             gs += 1
-            ahead.pop(0)
 
     def mma(self, me):
         gs = it = 0
@@ -205,4 +206,4 @@ def test_random_items(rules):
 @pytest.mark.parametrize("stages,items", [(2, [1, 0, 0, 0, 0]), (3, [1, 0, 0, 0, 0]), (3, [3, 0, 1, 0, 0, 1, 0, 0, 4])])
 def test_an_issuer_that_always_waits_for_the_next_item_waits_for_itself(rules, stages, items):
     with pytest.raises(Deadlock):
-        run_all(rules, items, stages, may_wait=lambda ahead: True)
+        run_all(rules, items, stages, may_wait=lambda converted, first: True)
