@@ -143,21 +143,23 @@ def test_converted_product_at_the_rule(dev, bR, items, K, N, pad):
     vals = torch.randint(0, 0x7f, (n, bR, 16), generator=g, device=dev, dtype=torch.uint8)
     vals ^= torch.randint(0, 2, (n, bR, 16), generator=g, device=dev, dtype=torch.uint8) << 7
     sc = torch.rand(n, generator=g, device=dev) * 0.02 + 1e-4
+    sc[::3] = torch.exp2(torch.randint(-12, 3, (len(sc[::3]),), generator=g, device=dev).float())   # subnormal in fp16
     t = lambda a: torch.from_numpy(np.ascontiguousarray(a.astype(np.int32))).to(dev)
     A = m.BCSR(MB * bR, K, bR, 16, t(np.concatenate([[0], np.cumsum(keep.sum(1))])), t(np.nonzero(keep)[1]),
                vals.view(-1), m.DType.E4M3, None, sc)
     Bw = torch.full((K, N + pad), 0x7f, dtype=torch.uint8, device=dev)
     Bw[:, :N] = torch.randint(0, 0x7f, (K, N), generator=g, device=dev, dtype=torch.uint8)
     C = torch.full((MB * bR, N), float("nan"), device=dev)
-    m.spmm(A, Bw[:, :N], N=N, C=C)
+    m.spmm(A, Bw[:, :N], N=N, C=C, b_scale=0.75)
     m.device_error_check()
     Ad = torch.zeros(MB, KB, bR, 16, dtype=torch.float64, device=dev)
     Ad[torch.from_numpy(keep).to(dev)] = (vals.view(torch.float8_e4m3fn).float() * sc[:, None, None]).half().double()
     Ad = Ad.permute(0, 2, 1, 3).reshape(MB * bR, K)
     Bd = Bw[:, :N].contiguous().view(torch.float8_e4m3fn).double()
     terms = t(16 * keep.sum(1)).double().repeat_interleave(bR)[:, None]
-    bound = terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs())
-    assert ((C.double() - Ad @ Bd).abs() <= bound).all()
+    ref = 0.75 * (Ad @ Bd)
+    bound = 0.75 * terms * 2.0 ** -23 * (Ad.abs() @ Bd.abs()) + 2.0 ** -24 * ref.abs()
+    assert ((C.double() - ref).abs() <= bound).all()
 
 
 @pytest.mark.parametrize("bR,N", [(16, 144), (16, 4096), (32, 128), (64, 272)])
